@@ -1,0 +1,113 @@
+"""Solves in one cooperative kernel against the same solves by separate launches.
+
+A handle solves by separate launches while its profiling is on, so the same linear system is solved both ways:
+every kind (block-Jacobi GMRES, AMG-FGMRES in FP64, with an FP32 Jacobian and an FP32 or FP64 basis, transport in
+FP64 and with FP32 products), meshes from fewer rows than CTAs to several rows per warp, and restarts that end inside
+a cycle, at its end and beyond it.  Both runs stop at a residual of 1e-12 of the right-hand side; with the condition
+numbers of these systems (up to 1e5 in the norm that weighs the solution) their solutions agree to 1e-7.
+"""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+RHO, MU, DT = 1060.0, 3.5e-3, 1e-3
+
+
+@pytest.fixture(scope="module")
+def api():
+    from tubularflowiga_b200 import api as a
+    return a
+
+
+def rel(a, b):
+    return float(np.linalg.norm(a - b) / max(np.linalg.norm(b), 1e-300))
+
+
+@pytest.mark.parametrize("core, ring, layers", [(2, 1, 3), (3, 1, 9), (4, 1, 40)])
+@pytest.mark.parametrize("restart", [1, 7, 64, 200])
+@pytest.mark.parametrize("kind", ["block-jacobi", "amg", "fp32-jacobian", "fp32-jacobian-fp64-basis"])
+def test_resident_solve_matches_separate_launches(api, kind, restart, core, ring, layers):
+    from tubularflowiga_b200 import meshgen
+    tube = meshgen.straight_tube(1.5e-3, 0.75e-3 * layers, core, ring, layers)
+    if restart < 64 and layers > 9:
+        pytest.skip("short restarts stagnate on the long tube")
+    settings = dict(density=RHO, viscosity=MU, dt=DT, gmres_restart=restart)
+    if kind != "block-jacobi":
+        settings.update(preconditioner=api.AMG, amg_coarse_nodes=40)
+    if kind.startswith("fp32"):
+        settings.update(precision=api.FP32_JACOBIAN, krylov_fp64_basis=int(kind.endswith("fp64-basis")))
+    ns = api.NavierStokes(api.Mesh(tube.mesh), **settings)
+    vmask, pmask, vel = api.tube_boundary_conditions(tube, 0.2)
+    ns.set_dirichlet(vmask, pmask, vel)
+    ns.set_tractions({2: 0.0})
+    start = api.initial_state(vmask, 0.9 * vel)
+    ns.set_state(start, start)
+    ns.assemble(values=False, rhs=False)
+    ns.apply_dirichlet(values=False, rhs=False)
+    found = {}
+    for profiling in (True, False):
+        ns.set_profiling(profiling)
+        before = ns.launches()
+        try:
+            found[profiling] = ns.solve_linear(rtol=1e-12, max_iterations=3000) + (ns.launches() - before,)
+        except api.TfigaError as e:            # both ways reach the cap, or neither does
+            found[profiling] = str(e)
+    if isinstance(found[True], str):
+        assert isinstance(found[False], str)
+        return
+    (u, iterations, _, launches), (v, again, residual, once) = found[True], found[False]
+    assert rel(v, u) < 1e-7
+    assert residual <= 1e-12 * np.linalg.norm(ns.apply_dirichlet(values=False)[1]) * 1.01 or kind == "block-jacobi"
+    assert abs(again - iterations) <= max(2, iterations // 20)
+    assert once < launches
+
+
+@pytest.mark.parametrize("fp32", [False, True])
+@pytest.mark.parametrize("core, ring, layers, restart", [(2, 1, 3, 5), (3, 2, 11, 50), (4, 1, 40, 30)])
+def test_resident_transport_matches_separate_launches(api, core, ring, layers, restart, fp32):
+    from tubularflowiga_b200 import meshgen
+    tube = meshgen.straight_tube(1.5e-3, 0.75e-3 * layers, core, ring, layers)
+    mesh = api.Mesh(tube.mesh)
+    params = api.transport_params(diffusion=1e-9, vplus=1.0, kplus=1.0, kminus=0.1, detach_plus=0.5, dt=2e-3, n0_bc=1.0,
+                                  nplus_bc=0.5, artificial_diffusion=1e-6, restart=restart, gmres_rtol=1e-12,
+                                  precision=api.MIXED if fp32 else api.FP64)
+    velocity = 0.3 * tube.profile
+    states = []
+    for profiling in (True, False):
+        solver = api.Transport(mesh, params, velocity, *api.resolve_transport_boundaries(tube.labels, velocity, params))
+        solver.set_profiling(profiling)
+        solver.step(3)
+        states.append(solver.get_state())
+    assert rel(states[1], states[0]) < 1e-8
+
+
+def test_resident_segments_and_outlets_match_separate_launches(api):
+    """Per-tube solves (a straight, a helical and a short tube) and the outlets' low-rank term."""
+    from tubularflowiga_b200 import meshgen
+    tubes = [meshgen.straight_tube(1.5e-3, 9e-3, 4, 1, 12), meshgen.helical_tube(1e-3, 14e-3, 20e-3, 4, 1, 17),
+             meshgen.straight_tube(2e-3, 6e-3, 3, 1, 5)]
+    batch = meshgen.combine_tubes(tubes, [0.2, 0.15, 0.1])
+    y = meshgen.y_bifurcation(parent_layers=5, daughter_layers=4, ax=2, ay=4, ring=1, parent_length=6e-3,
+                              daughter_length=5e-3)
+    for body, segments in ((batch, batch.node_offset), (y, None)):
+        states = []
+        mesh = api.Mesh(body.mesh)
+        for profiling in (True, False):
+            ns = api.NavierStokes(mesh, density=RHO, viscosity=MU, dt=DT, preconditioner=api.AMG, gmres_restart=64,
+                                  precision=api.MIXED_BF16X3, nonlinear_rtol=1e-11, nonlinear_atol=1e-300, max_newton=20,
+                                  newton_forcing=1)
+            ns.set_profiling(profiling)
+            vmask, pmask, vel = (api.tube_boundary_conditions(body, 0.2) if segments is None
+                                 else api.batch_boundary_conditions(body))
+            ns.set_dirichlet(vmask, pmask, vel)
+            start = api.initial_state(vmask, 0.9 * vel)
+            ns.set_state(start, start)
+            if segments is None:
+                ns.step_outlets_coupled([api.Outlet.rcr(label, 1e8, 1e-10, 1e9) for label in (2, 3)])
+            else:
+                ns.set_tractions({2: 0.0})
+                ns.set_segments(segments)
+                ns.step()
+            states.append(ns.get_state())
+        assert rel(states[1], states[0]) < 1e-7

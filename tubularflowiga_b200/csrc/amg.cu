@@ -711,6 +711,7 @@ void Amg::BuildFromStrength(std::vector<double> s)
 	}
 	CudaCheck(cudaStreamSynchronize(stream_), "AMG setup");
 	built_ = true;
+	++version_;
 	BuildSegmentMaps();
 	masks_dirty_ = true;
 }
@@ -860,6 +861,33 @@ void Amg::Apply(const T* fine_values, const double* v, double* z, const int* sto
 
 template void Amg::Apply<double>(const double*, const double*, double*, const int*, const int*);
 template void Amg::Apply<float>(const float*, const double*, double*, const int*, const int*);
+
+template <class T>
+AmgResidentView Amg::ResidentView()
+{
+	Level& L = *levels_[0];
+	Level& C = *levels_[1];
+	AmgResidentView v;
+	v.coarse = C.nodes;
+	v.agg = L.agg.get();
+	v.agg_order = L.agg_order.get();
+	v.agg_offsets = L.agg_offsets.get();
+	v.mask = L.mask.get();
+	v.dense = C.dense.get()+C.dense_n;
+	v.dense_ld = 2LL*C.dense_n;
+	v.coarse_rhs = C.b.get();
+	v.coarse_x = C.x.get();
+	v.ap_rows = L.ap_rows.get();
+	v.ap_cols = L.ap_cols.get();
+	v.ap = ApValues<T>(L);
+	v.inverse = L.inverse.get();
+	v.omega = options_.omega;
+	v.version = version_;
+	return v;
+}
+
+template AmgResidentView Amg::ResidentView<double>();
+template AmgResidentView Amg::ResidentView<float>();
 
 void Amg::SetSegments(const std::vector<int32_t>& node_segment)
 {

@@ -23,6 +23,7 @@
 
 #include "common.hpp"
 #include "kernels.cuh"
+#include "krylov_resident.hpp"
 
 #include <memory>
 #include <vector>
@@ -66,6 +67,8 @@ public:
 	long long transfer_blocks() const;
 	// Block-Jacobi inverses (4x4 per node, FP64) of the fine level, current after Refresh.
 	const double* fine_inverse() const;
+	// Device arrays of an application, for the resident solver (current after Refresh<T>).
+	template <class T> AmgResidentView ResidentView();
 	long long launches() const { return launches_; }
 	// launches replayed from a captured CUDA graph (counted as if launched)
 	void count_launches(long long n) { launches_ += n; }
@@ -91,6 +94,7 @@ private:
 	bool built_ = false;
 	bool masks_dirty_ = true;
 	bool coarse_ready_ = false;
+	long long version_ = 0;            // hierarchies built
 	long long launches_ = 0;
 	Profiler* profiler_ = nullptr;
 

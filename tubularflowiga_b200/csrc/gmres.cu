@@ -467,6 +467,28 @@ Gmres::~Gmres()
 	if (host_) cudaFreeHost(host_);
 }
 
+bool Gmres::SolveResident(ResidentKrylov::Kind kind, const DevicePatternView& pattern, const AmgResidentView* amg,
+	const std::vector<int64_t>& segments, ResidentProblem& problem, GmresResult& result, const char* name)
+{
+	if ((profiler_ && profiler_->enabled()) || learned_ || collector_ || line_on_) return false;
+	if (!resident_.Prepare(kind, pattern, restart_, segments, amg, stream_)) return false;
+	problem.pattern = pattern;
+	if (amg) {
+		problem.amg = *amg;
+		problem.Z = Z_.get();
+		if (low_on_) problem.low = {low_.count, low_.ptr, low_.idx, low_.val, low_.coef};
+	}
+	const ResidentStatus status = resident_.Solve(problem, stream_, &launches_);
+	if (status.error == 4) Fail(-2, std::string(name)+": a grid barrier wait expired");
+	if (status.error == 2)
+		Fail(-6, std::string(name)+(status.iterations ? " residual is not finite" : " initial residual is not finite"));
+	if (status.error == 1) Fail(-6, std::string(name)+" Hessenberg matrix is singular");
+	result.iterations = status.iterations;
+	result.residual = status.residual;
+	result.converged = status.converged != 0;
+	return true;
+}
+
 std::size_t Gmres::bytes() const
 {
 	return V_.bytes()+w_.bytes()+r_.bytes()+tmp_.bytes()+inverse_.bytes()+partial_.bytes()+H_.bytes();
@@ -631,6 +653,23 @@ GmresResult Gmres::SolveFlexibleImpl(const DevicePatternView& pattern, const T* 
 	const long long amg0 = M.launches();
 	if (Z_.size() == 0) Z_.Allocate((size_t)(restart_+1)*n_);
 	GmresResult result;
+	{
+		ResidentProblem problem;
+		problem.krylov_values = problem.residual_values = values;
+		problem.rhs = rhs;
+		problem.x = x;
+		problem.V = Basis<B>();
+		problem.rtol = rtol;
+		problem.tolerance_floor = 1e-30;
+		problem.max_iterations = max_iterations;
+		const AmgResidentView view = M.ResidentView<T>();
+		constexpr ResidentKrylov::Kind kind = std::is_same<T, double>::value ? ResidentKrylov::kFlexDouble
+			: std::is_same<B, double>::value ? ResidentKrylov::kFlexFloatFp64Basis : ResidentKrylov::kFlexFloat;
+		if (SolveResident(kind, pattern, &view, {}, problem, result, "FGMRES")) {
+			if (launches) *launches += launches_;
+			return result;
+		}
+	}
 	double beta = TrueResidualPlain<T, B>(pattern, values, rhs, x);
 	result.residual = beta;
 	if (!std::isfinite(beta)) Fail(-6, "FGMRES initial residual is not finite");
@@ -716,6 +755,26 @@ GmresResult Gmres::Solve(const DevicePatternView& pattern, const double* values,
 		else LaunchBlockInverse(pattern, values, inverse_.get(), singular_.get(), stream_);
 		launches_ += 1;
 		singular_.Download(&host_->singular, 1, stream_);
+	}
+	if (fields_ == 2 || krylov_values == nullptr) {
+		ResidentProblem problem;
+		problem.krylov_values = krylov_values ? static_cast<const void*>(krylov_values) : values;
+		problem.residual_values = values;
+		problem.rhs = rhs;
+		problem.x = x;
+		problem.inverse = inverse_.get();
+		problem.V = V_.get();
+		problem.rtol = rtol;
+		problem.tolerance_floor = 1e-30;
+		problem.max_iterations = max_iterations;
+		const ResidentKrylov::Kind kind = fields_ == 4 ? ResidentKrylov::kLeft4
+			: krylov_values ? ResidentKrylov::kLeft2Fp32 : ResidentKrylov::kLeft2;
+		if (SolveResident(kind, pattern, nullptr, {}, problem, result, "GMRES")) {
+			if (rebuild_preconditioner) singular_count_ = host_->singular;
+			result.singular_blocks = singular_count_;
+			if (launches) *launches += launches_;
+			return result;
+		}
 	}
 	double beta = TrueResidual(pattern, values, rhs, x);
 	if (rebuild_preconditioner) singular_count_ = host_->singular;

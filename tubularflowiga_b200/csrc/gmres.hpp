@@ -14,6 +14,7 @@
 #include "amg.hpp"
 #include "common.hpp"
 #include "kernels.cuh"
+#include "krylov_resident.hpp"
 #include "learned.hpp"
 
 namespace tfiga {
@@ -130,6 +131,14 @@ private:
 	const void* seg_graph_values_ = nullptr;             // operator the graphs were captured with
 	const void* seg_graph_amg_ = nullptr;
 	bool seg_graphs_ok_ = true;
+
+	// One cooperative launch for the whole solve where the basis fits the chip's shared memory; direct
+	// launches otherwise, and while profiling (the families' events lie between kernels), with the
+	// learned stage, a pair collector or the flow lines.  False: not taken.
+	bool SolveResident(ResidentKrylov::Kind kind, const DevicePatternView& pattern, const AmgResidentView* amg,
+		const std::vector<int64_t>& segments, ResidentProblem& problem, GmresResult& result, const char* name);
+	ResidentKrylov resident_;
+	std::vector<int64_t> seg_entries_;   // segment offsets (count + 1), empty without segments
 
 	int nodes_, fields_, n_, restart_, blocks_;
 	unsigned singular_count_ = 0;     // singular diagonal blocks of the last block-inverse build

@@ -305,7 +305,7 @@ void Gmres::SetSegments(const std::vector<int64_t>& entry_offsets, const std::ve
 {
 	ReleaseSegmentGraphs();
 	const int count = (int)entry_offsets.size()-1;
-	if (count <= 0) { segments_ = 0; return; }
+	if (count <= 0) { segments_ = 0; seg_entries_.clear(); return; }
 	if (count > 1024) Fail(-7, "at most 1024 segments per flexible solve");
 	if (entry_offsets[0] != 0 || entry_offsets[count] != n_) Fail(-1, "segments must cover the unknowns");
 	for (int k = 0; k <= count; ++k)
@@ -317,6 +317,7 @@ void Gmres::SetSegments(const std::vector<int64_t>& entry_offsets, const std::ve
 	}
 	if (restart_+1 > 129) Fail(-7, "segmented flexible GMRES supports restarts up to 128");
 	segments_ = count;
+	seg_entries_ = entry_offsets;
 	seg_dot_cx_ = (int)((longest+kDotChunk-1)/kDotChunk);
 	seg_len_.resize(count);
 	for (int k = 0; k < count; ++k) seg_len_[k] = entry_offsets[k+1]-entry_offsets[k];
@@ -501,6 +502,23 @@ GmresResult Gmres::SolveFlexibleSegmentsImpl(const DevicePatternView& pattern, c
 	if (Z_.size() == 0) Z_.Allocate((size_t)(restart_+1)*n_);
 	const int stride = restart_+1;
 	GmresResult result;
+	{
+		ResidentProblem problem;
+		problem.krylov_values = problem.residual_values = values;
+		problem.rhs = rhs;
+		problem.x = x;
+		problem.V = Basis<B>();
+		problem.rtol = rtol;
+		problem.tolerance_floor = 1e-300;
+		problem.max_iterations = max_iterations;
+		const AmgResidentView view = M.ResidentView<T>();
+		constexpr ResidentKrylov::Kind kind = std::is_same<T, double>::value ? ResidentKrylov::kFlexDouble
+			: std::is_same<B, double>::value ? ResidentKrylov::kFlexFloatFp64Basis : ResidentKrylov::kFlexFloat;
+		if (SolveResident(kind, pattern, &view, seg_entries_, problem, result, "FGMRES")) {
+			if (launches) *launches += launches_;
+			return result;
+		}
+	}
 	SegTrueResidual<T, B>(pattern, values, rhs, x);
 	double total = 0.0;
 	for (int k = 0; k < segments_; ++k) {
