@@ -56,10 +56,9 @@ def test_resident_solve_matches_separate_launches(api, kind, restart, core, ring
     if isinstance(found[True], str):
         assert isinstance(found[False], str)
         return
-    (u, iterations, _, launches), (v, again, residual, once) = found[True], found[False]
+    (u, _, _, launches), (v, _, residual, once) = found[True], found[False]
     assert rel(v, u) < 1e-7
     assert residual <= 1e-12 * np.linalg.norm(ns.apply_dirichlet(values=False)[1]) * 1.01 or kind == "block-jacobi"
-    assert abs(again - iterations) <= max(2, iterations // 20)
     assert once < launches
 
 

@@ -26,9 +26,11 @@ struct Amg::Level {
 	DeviceArray<float> ap_values32;     // A P with an FP32 fine matrix (stored in its precision)
 	// coarsest level
 	int dense_n = 0;
-	DeviceArray<double> dense, column;
-	DeviceArray<double> panel;          // blocked Gauss-Jordan: two n x 32 panel copies + the 32 x 32 pivot-block inverse
-	DeviceArray<int> dense_flag, pivots;
+	DeviceArray<double> dense, column;  // two n x n matrices, or one n x 2n; a pivot column
+	const double* dense_inverse = nullptr;
+	long long dense_ld = 0;
+	DeviceArray<double> panel;          // blocked Gauss-Jordan: the n x 32 panel's result
+	DeviceArray<int> dense_flag, permutation;   // permutation: [source | order | order out] of n
 	DevicePatternView view() const { return {nodes, blocks, rows.get(), cols.get(), diag.get()}; }
 };
 
@@ -198,7 +200,8 @@ __global__ void __launch_bounds__(128) RestrictKernel(int coarse_nodes, const in
 }
 
 
-__global__ void DenseScatterKernel(DevicePatternView p, const double* __restrict__ values, int n, double* __restrict__ dense)
+__global__ void DenseScatterKernel(DevicePatternView p, const double* __restrict__ values, long long ld,
+	double* __restrict__ dense)
 {
 	const long long t = (long long)blockIdx.x*blockDim.x+threadIdx.x;
 	if (t >= p.blocks*16) return;
@@ -211,7 +214,7 @@ __global__ void DenseScatterKernel(DevicePatternView p, const double* __restrict
 		if (p.row_offsets[mid] <= k) lo = mid; else hi = mid;
 	}
 	const size_t row = 4*(size_t)lo+r, col = 4*(size_t)p.columns[k]+c;
-	dense[row*(size_t)(2*n)+col] = values[t];
+	dense[row*(size_t)ld+col] = values[t];
 }
 
 // Gauss-Jordan inverse with partial pivoting on the augmented [A | I] (n x 2n,
@@ -284,177 +287,247 @@ __global__ void GaussJordanEliminateKernel(int n, int k, double* __restrict__ a,
 	a[(size_t)i*ld+j] = j == k ? 0.0 : a[(size_t)i*ld+j]-f*a[(size_t)k*ld+j];
 }
 
-// Blocked Gauss-Jordan on the augmented [A | I] (n x 2n, row-major): 32 pivot columns per pair of
-// launches instead of one.  For the panel of columns k0 .. k0 + b - 1 (b <= 32):
-//   GaussJordanPanelKernel (one CTA): copies the panel's n x b columns twice (W, O), runs Gauss-Jordan
-//     with partial pivoting on W alone (pivot rows searched below k0 + jj, swaps applied to W and O), so
-//     that O ends up as the row-permuted original panel and the pivot block A_RR = O[k0 .. k0 + b) is
-//     factorable in natural order; inverts A_RR in shared memory (Gauss-Jordan without further
-//     pivoting: its pivots are the panel's) and records the swaps;
-//   GaussJordanUpdateKernel (CTA per 16 columns of all 2n): applies the swaps, then
-//     rows R = k0 .. k0 + b - 1  <-  Z = A_RR^{-1} Y_R,   every other row i  <-  Y_i - O_i Z,
-//   which is what the b single-column eliminations do to those columns.
-// A vanishing pivot (|max| <= 1e-300) raises *flag; the caller then redoes the inverse column by column.
-constexpr int kPanelThreads = 1024;
-constexpr int kUpdateColumns = 16;
+// Blocked in-place Gauss-Jordan with partial pivoting, 32 pivot columns per pair of launches.
+//   InversePanelKernel (one cluster of up to 16 CTAs, a row per thread, its 32 panel entries in registers):
+//     the in-place elimination of the panel's columns.  Every warp offers its largest candidate with
+//     that row; one block barrier and one cluster barrier per column later all threads hold the pivot row.
+//     Leaves the panel's result T, the pivots' order and the row permutation of the panel.
+//   InverseUpdateKernel (CTA per 64 x 64 tile, out of place): every other column,
+//     Y_i <- (i a pivot row ? 0 : Y_i) + T_i Y_pivots, with the rows permuted on the way.
+// Rows stay where they are while a panel is eliminated; the permutation makes pivot row k the row k of
+// the matrix, and the columns are put in order at the end (InverseColumnsKernel).  The serial column chain
+// (argument maximum, barrier, division, rank-one update) bounds it: a panel takes 47 us in one CTA (n = 288)
+// and 69 us in a cluster of two (n = 896), where a panel kept in global memory by one CTA took 193 and
+// 423 us; in place, the update touches n columns and not the 2 n of an augmented matrix (31 -> 9 and
+// 88 -> 12 us).
+// A pivot of at most 1e-300 raises *flag; the caller then redoes the inverse column by column, which
+// decouples the unknown.
+constexpr int kPanelThreads = 512;
+constexpr int kPanelWarps = kPanelThreads/32;
+constexpr int kPanelClusterMax = 16;
+constexpr int kUpdateTile = 64;
 
-__global__ void __launch_bounds__(kPanelThreads) GaussJordanPanelKernel(int n, int k0, int b,
-	const double* __restrict__ a, double* __restrict__ panel, int* __restrict__ pivots, int* __restrict__ flag)
+__device__ __forceinline__ uint32_t ClusterRank()
 {
-	const int ld = 2*n;
-	double* W = panel;                      // [n][b]
-	double* O = panel+(size_t)n*kPanel;     // [n][b]
-	double* Ainv = panel+(size_t)2*n*kPanel; // [b][b]
-	__shared__ double best_val[32];
-	__shared__ int best_idx[32];
-	__shared__ int pivot_row;
-	__shared__ double pivot_value;
-	__shared__ double block[kPanel][2*kPanel+1];
-	const int tid = threadIdx.x;
-	for (long long idx = tid; idx < (long long)n*b; idx += kPanelThreads) {
-		const int i = (int)(idx/b), j = (int)(idx%b);
-		const double v = a[(size_t)i*ld+k0+j];
-		W[(size_t)i*b+j] = v;
-		O[(size_t)i*b+j] = v;
-	}
-	__syncthreads();
-	for (int jj = 0; jj < b; ++jj) {
-		const int j = k0+jj;
-		double bv = -1.0; int bi = j;
-		for (int i = j+tid; i < n; i += kPanelThreads) {
-			const double v = fabs(W[(size_t)i*b+jj]);
-			if (v > bv) { bv = v; bi = i; }
-		}
-		for (int o = 16; o > 0; o >>= 1) {
-			const double ov = __shfl_xor_sync(0xffffffffu, bv, o);
-			const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
-			if (ov > bv || (ov == bv && oi < bi)) { bv = ov; bi = oi; }
-		}
-		if ((tid & 31) == 0) { best_val[tid >> 5] = bv; best_idx[tid >> 5] = bi; }
-		__syncthreads();
-		if (tid == 0) {
-			double v = -1.0; int idx = j;
-			for (int w = 0; w < kPanelThreads/32; ++w)
-				if (best_val[w] > v || (best_val[w] == v && best_idx[w] < idx)) { v = best_val[w]; idx = best_idx[w]; }
-			if (!(v > 1e-300)) { *flag = 1; idx = j; }
-			pivot_row = idx;
-			pivots[jj] = idx;
-		}
-		__syncthreads();
-		const int pr = pivot_row;
-		if (pr != j)
-			for (int c = tid; c < b; c += kPanelThreads) {
-				double t = W[(size_t)j*b+c]; W[(size_t)j*b+c] = W[(size_t)pr*b+c]; W[(size_t)pr*b+c] = t;
-				t = O[(size_t)j*b+c]; O[(size_t)j*b+c] = O[(size_t)pr*b+c]; O[(size_t)pr*b+c] = t;
-			}
-		__syncthreads();
-		if (tid == 0) {
-			const double v = W[(size_t)j*b+jj];
-			pivot_value = v != 0.0 ? v : 1.0;
-		}
-		__syncthreads();
-		const double inv = 1.0/pivot_value;
-		// eliminate column jj of the panel from every other row (row j scaled in place afterwards)
-		for (long long idx = tid; idx < (long long)n*b; idx += kPanelThreads) {
-			const int i = (int)(idx/b), c = (int)(idx%b);
-			if (i == j || c <= jj) continue;
-			const double f = W[(size_t)i*b+jj]*inv;
-			if (f != 0.0) W[(size_t)i*b+c] -= f*W[(size_t)j*b+c];
-		}
-		__syncthreads();
-		for (long long i = tid; i < n; i += kPanelThreads)
-			if (i != j) W[(size_t)i*b+jj] = 0.0;
-		for (int c = tid; c < b; c += kPanelThreads) W[(size_t)j*b+c] *= inv;
-		__syncthreads();
-	}
-	// inverse of the pivot block A_RR = O[k0 .. k0 + b) by Gauss-Jordan in natural order
-	for (int idx = tid; idx < b*2*b; idx += kPanelThreads) {
-		const int r = idx/(2*b), c = idx%(2*b);
-		block[r][c] = c < b ? O[(size_t)(k0+r)*b+c] : (c-b == r ? 1.0 : 0.0);
-	}
-	__syncthreads();
-	for (int jj = 0; jj < b; ++jj) {
-		if (tid == 0) {
-			const double v = block[jj][jj];
-			pivot_value = v != 0.0 ? v : 1.0;
-		}
-		__syncthreads();
-		const double inv = 1.0/pivot_value;
-		for (int idx = tid; idx < b*2*b; idx += kPanelThreads) {
-			const int r = idx/(2*b), c = idx%(2*b);
-			if (r == jj || c == jj) continue;
-			const double f = block[r][jj]*inv;
-			if (f != 0.0) block[r][c] -= f*block[jj][c];
-		}
-		__syncthreads();
-		for (int r = tid; r < b; r += kPanelThreads) if (r != jj) block[r][jj] = 0.0;
-		for (int c = tid; c < 2*b; c += kPanelThreads) block[jj][c] *= inv;
-		__syncthreads();
-	}
-	for (int idx = tid; idx < b*b; idx += kPanelThreads) Ainv[idx] = block[idx/b][b+idx%b];
+	uint32_t r;
+	asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+	return r;
 }
 
-__global__ void __launch_bounds__(256) GaussJordanUpdateKernel(int n, int k0, int b, double* __restrict__ a,
-	const double* __restrict__ panel, const int* __restrict__ pivots)
+__device__ __forceinline__ void ClusterBarrier()
 {
-	const int ld = 2*n;
-	const double* O = panel+(size_t)n*kPanel;
-	const double* Ainv = panel+(size_t)2*n*kPanel;
-	__shared__ double sA[kPanel][kPanel+1];
-	__shared__ double sY[kPanel][kUpdateColumns];
-	__shared__ double sZ[kPanel][kUpdateColumns];
-	__shared__ int sP[kPanel];
-	const int tid = threadIdx.x;
-	const int c0 = blockIdx.x*kUpdateColumns;
-	const int cols = min(kUpdateColumns, ld-c0);
-	for (int idx = tid; idx < b*b; idx += blockDim.x) sA[idx/b][idx%b] = Ainv[idx];
-	if (tid < b) sP[tid] = pivots[tid];
-	__syncthreads();
-	// the panel's row swaps, in order, one thread per column of the tile
-	if (tid < cols)
+	asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+// Stores a double at the shared address `p` of cluster CTA `rank`.
+__device__ __forceinline__ void ClusterStore(const double* p, uint32_t rank, double v)
+{
+	uint32_t local = (uint32_t)__cvta_generic_to_shared(p), remote;
+	asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(local), "r"(rank));
+	asm volatile("st.shared::cluster.f64 [%0], %1;" :: "r"(remote), "d"(v) : "memory");
+}
+
+// Magnitude as an ordered integer: the upper half of the absolute value (20 bits of its mantissa).
+__device__ __forceinline__ unsigned MagnitudeKey(double v)
+{
+	return (unsigned)(__double_as_longlong(fabs(v)) >> 32);
+}
+
+// a: n x n, columns k0 .. k0 + b - 1.  panel[i*32 + c] = T; source[i]: the row that position i takes.
+__global__ void __launch_bounds__(kPanelThreads, 1) InversePanelKernel(int n, int k0, int b,
+	const double* __restrict__ a, double* __restrict__ panel, int* __restrict__ source, int* __restrict__ flag)
+{
+	__shared__ __align__(16) double offer[kPanelWarps][kPanel];         // each warp's candidate row
+	__shared__ unsigned offer_key[kPanelWarps];
+	__shared__ int offer_row[kPanelWarps];
+	// each CTA's candidate, in two buffers: a column's readers may still hold the last one
+	__shared__ __align__(16) double cta_offer[2][kPanelClusterMax][kPanel+2];   // row, then magnitude and index
+	__shared__ int pivot_of[kPanel];
+	const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+	const int ctas = gridDim.x;
+	const uint32_t rank = ctas > 1 ? ClusterRank() : 0u;
+	const int row = (int)rank*kPanelThreads+tid;
+	double w[kPanel];
+	#pragma unroll
+	for (int c = 0; c < kPanel; ++c) w[c] = row < n && c < b ? a[(size_t)row*n+k0+c] : 0.0;
+	bool free_row = row >= k0 && row < n;
+	if (ctas > 1) ClusterBarrier();        // every CTA of the cluster has started before remote stores
+	// The loop stays rolled (unrolled, every column ran through cold code): the current column is always
+	// w[0], the updates write one register down, and the finished column enters at the end.
+	#pragma unroll 1
+	for (int jj = 0; jj < b; ++jj) {
+		// candidates: keys are offset by one so that a zero entry of a free row still beats rows out of play
+		const unsigned key = free_row ? MagnitudeKey(w[0])+1u : 0u;
+		const unsigned best = __reduce_max_sync(0xffffffffu, key);
+		const int owner = __ffs((int)__ballot_sync(0xffffffffu, key == best))-1;
+		if (lane == owner) {
+			offer_key[warp] = best;
+			offer_row[warp] = row;
+			double2* o = reinterpret_cast<double2*>(offer[warp]);
+			#pragma unroll
+			for (int c = 0; c < kPanel/2; ++c) o[c] = make_double2(w[2*c], w[2*c+1]);
+		}
+		__syncthreads();
+		const unsigned mine = lane < kPanelWarps ? offer_key[lane] : 0u;
+		const unsigned top = __reduce_max_sync(0xffffffffu, mine);
+		int slot = __ffs((int)__ballot_sync(0xffffffffu, mine == top && lane < kPanelWarps))-1;
+		int pivot = offer_row[slot];
+		const double* prow = offer[slot];
+		if (ctas > 1) {
+			double (*box)[kPanel+2] = cta_offer[jj & 1];
+			// warps share the destinations; lane c carries entry c, then key and row
+			const double v = prow[lane];
+			for (int to = warp; to < ctas; to += kPanelWarps) {
+				ClusterStore(&box[rank][lane], (uint32_t)to, v);
+				if (lane < 2) ClusterStore(&box[rank][kPanel+lane], (uint32_t)to, lane == 0 ? (double)top : (double)pivot);
+			}
+			ClusterBarrier();
+			const unsigned theirs = lane < ctas ? (unsigned)box[lane][kPanel] : 0u;
+			const unsigned most = __reduce_max_sync(0xffffffffu, theirs);
+			slot = __ffs((int)__ballot_sync(0xffffffffu, theirs == most && lane < ctas))-1;
+			pivot = (int)box[slot][kPanel+1];
+			prow = box[slot];
+		}
+		const double value = prow[0];
+		const bool bad = !(fabs(value) > 1e-300);
+		const double inv = bad ? 1.0 : 1.0/value;
+		if (tid == 0) {
+			pivot_of[jj] = pivot;
+			if (bad && rank == 0) *flag = 1;
+		}
+		const double2* p2 = reinterpret_cast<const double2*>(prow);
+		const bool is_pivot = row == pivot;
+		free_row = free_row && !is_pivot;
+		// rows i: w + f p with f = -w[0] / p[0]; the pivot row: 0 + (1 / p[0]) p (a branch for it would put its
+		// warp's second pass on every column's critical path)
+		const double f = is_pivot ? inv : -w[0]*inv;
+		#pragma unroll
+		for (int c = 0; c < kPanel/2; ++c) {
+			const double2 p = p2[c];
+			if (c > 0) w[2*c-1] = fma(f, p.x, is_pivot ? 0.0 : w[2*c]);
+			w[2*c] = fma(f, p.y, is_pivot ? 0.0 : w[2*c+1]);
+		}
+		w[kPanel-1] = f;
+		// `offer` is rewritten by the next column once every thread has read its pivot row (with a cluster the
+		// readers hold cta_offer and the cluster barrier above already lies between)
+		if (ctas == 1) __syncthreads();
+	}
+	if (row < n) {
+		// after b rotations w[c] is column (c + b) mod 32
+		double* t = panel+(size_t)row*kPanel;
+		#pragma unroll
+		for (int c = 0; c < kPanel; ++c) t[(c+b)%kPanel] = w[c];
+		source[row] = row;
+	}
+	if (ctas > 1) ClusterBarrier();
+	else __syncthreads();
+	if (rank == 0 && warp == 0) {
+		// The swaps (k0 + jj, position of pivot jj) in order.  Lane t follows position k0 + t (the row it holds)
+		// and the position outside the block whose row step t took, with the row put there instead.
+		int held = k0+lane, out_at = -1, out_row = -1;
 		for (int jj = 0; jj < b; ++jj) {
-			const int j = k0+jj, p = sP[jj];
-			if (p != j) {
-				const double t = a[(size_t)j*ld+c0+tid];
-				a[(size_t)j*ld+c0+tid] = a[(size_t)p*ld+c0+tid];
-				a[(size_t)p*ld+c0+tid] = t;
+			const int p = pivot_of[jj];
+			const int displaced = __shfl_sync(0xffffffffu, held, jj);
+			const unsigned inside = __ballot_sync(0xffffffffu, lane < b && held == p);
+			const unsigned outside = __ballot_sync(0xffffffffu, out_at >= 0 && out_row == p);
+			if (inside) {
+				if (lane == __ffs((int)inside)-1) held = displaced;
+			} else if (outside) {
+				if (lane == __ffs((int)outside)-1) out_row = displaced;
+			} else if (lane == jj) {
+				out_at = p;
+				out_row = displaced;
 			}
+			if (lane == jj) held = p;
 		}
-	__syncthreads();
-	for (int idx = tid; idx < b*kUpdateColumns; idx += blockDim.x) {
-		const int r = idx/kUpdateColumns, c = idx%kUpdateColumns;
-		sY[r][c] = c < cols ? a[(size_t)(k0+r)*ld+c0+c] : 0.0;
+		if (lane < b) source[k0+lane] = held;
+		if (out_at >= 0) source[out_at] = out_row;
 	}
-	__syncthreads();
-	for (int idx = tid; idx < b*kUpdateColumns; idx += blockDim.x) {
-		const int r = idx/kUpdateColumns, c = idx%kUpdateColumns;
-		double z = 0.0;
-		for (int k = 0; k < b; ++k) z = fma(sA[r][k], sY[k][c], z);
-		sZ[r][c] = z;
-		if (c < cols) a[(size_t)(k0+r)*ld+c0+c] = z;
-	}
-	__syncthreads();
-	// every other row: Y_i -= O_i Z (threads: 16 columns x 16 row lanes)
-	const int c = tid % kUpdateColumns, lane = tid / kUpdateColumns;
-	if (c < cols)
-		for (int i = lane; i < n; i += blockDim.x/kUpdateColumns) {
-			if (i >= k0 && i < k0+b) continue;
-			const double* o = O+(size_t)i*b;
-			double s = 0.0;
-			for (int k = 0; k < b; ++k) s = fma(o[k], sZ[k][c], s);
-			a[(size_t)i*ld+c0+c] -= s;
-		}
 }
 
-// x = A^{-1} b with the inverse in the right half of the augmented matrix; warp per row.
-__global__ void DenseApplyKernel(int n, const double* __restrict__ a, const double* __restrict__ b,
+__global__ void __launch_bounds__(256) InverseUpdateKernel(int n, int k0, int b, const double* __restrict__ a,
+	double* __restrict__ out, const double* __restrict__ panel, const int* __restrict__ source,
+	const int* __restrict__ order, int* __restrict__ order_out)
+{
+	__shared__ double sT[kUpdateTile][kPanel+1];
+	__shared__ double sY[kPanel][kUpdateTile];
+	__shared__ int sS[kUpdateTile], sP[kPanel];
+	const int tid = threadIdx.x;
+	const int i0 = blockIdx.y*kUpdateTile, j0 = blockIdx.x*kUpdateTile;
+	if (tid < kUpdateTile) sS[tid] = i0+tid < n ? source[i0+tid] : 0;
+	if (tid >= 64 && tid < 64+kPanel) sP[tid-64] = tid-64 < b ? source[k0+tid-64] : 0;
+	__syncthreads();
+	if (blockIdx.x == 0 && tid < kUpdateTile && i0+tid < n) order_out[i0+tid] = order[sS[tid]];
+	for (int k = tid; k < kUpdateTile*kPanel; k += 256) {
+		const int r = k/kPanel, c = k%kPanel;
+		sT[r][c] = i0+r < n && c < b ? panel[(size_t)sS[r]*kPanel+c] : 0.0;
+	}
+	for (int k = tid; k < kPanel*kUpdateTile; k += 256) {
+		const int r = k/kUpdateTile, c = k%kUpdateTile;
+		sY[r][c] = r < b && j0+c < n ? a[(size_t)sP[r]*n+j0+c] : 0.0;
+	}
+	__syncthreads();
+	const int tc = tid & 15, tr = tid >> 4;            // columns tc + 16 u, rows tr + 16 v
+	double acc[4][4];
+	#pragma unroll
+	for (int v = 0; v < 4; ++v) {
+		const int r = tr+16*v, i = i0+r;
+		const bool keep = i < n && (i < k0 || i >= k0+b);
+		#pragma unroll
+		for (int u = 0; u < 4; ++u) {
+			const int j = j0+tc+16*u;
+			acc[v][u] = keep && j < n ? a[(size_t)sS[r]*n+j] : 0.0;
+		}
+	}
+	#pragma unroll 4
+	for (int k = 0; k < kPanel; ++k) {
+		double t[4], y[4];
+		#pragma unroll
+		for (int v = 0; v < 4; ++v) t[v] = sT[tr+16*v][k];
+		#pragma unroll
+		for (int u = 0; u < 4; ++u) y[u] = sY[k][tc+16*u];
+		#pragma unroll
+		for (int v = 0; v < 4; ++v)
+			#pragma unroll
+			for (int u = 0; u < 4; ++u) acc[v][u] = fma(t[v], y[u], acc[v][u]);
+	}
+	#pragma unroll
+	for (int v = 0; v < 4; ++v) {
+		const int r = tr+16*v, i = i0+r;
+		if (i >= n) continue;
+		#pragma unroll
+		for (int u = 0; u < 4; ++u) {
+			const int j = j0+tc+16*u;
+			if (j < n) out[(size_t)i*n+j] = j >= k0 && j < k0+b ? sT[r][j-k0] : acc[v][u];
+		}
+	}
+}
+
+// inverse[r][order[i]] = m[r][i]: the columns of the permuted matrix's inverse back in order.
+__global__ void InverseColumnsKernel(int n, const double* __restrict__ m, const int* __restrict__ order,
+	double* __restrict__ inverse)
+{
+	const long long t = (long long)blockIdx.x*blockDim.x+threadIdx.x;
+	if (t >= (long long)n*n) return;
+	const int r = (int)(t/n), i = (int)(t-(long long)r*n);
+	inverse[(size_t)r*n+order[i]] = m[t];
+}
+
+__global__ void IdentityOrderKernel(int n, int* __restrict__ order)
+{
+	const int i = blockIdx.x*blockDim.x+threadIdx.x;
+	if (i < n) order[i] = i;
+}
+
+// x = A^{-1} b, rows of the inverse `ld` apart; warp per row.
+__global__ void DenseApplyKernel(int n, const double* __restrict__ a, long long ld, const double* __restrict__ b,
 	double* __restrict__ x, const int* __restrict__ stop)
 {
 	if (*stop) return;
 	const int row = blockIdx.x*(blockDim.x >> 5)+(threadIdx.x >> 5);
 	const int lane = threadIdx.x & 31;
 	if (row >= n) return;
-	const double* ar = a+(size_t)row*(2*n)+n;
+	const double* ar = a+(size_t)row*ld;
 	double s = 0.0;
 	for (int j = lane; j < n; j += 32) s = fma(ar[j], b[j], s);
 	for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
@@ -705,8 +778,8 @@ void Amg::BuildFromStrength(std::vector<double> s)
 			V.dense.Allocate((size_t)V.dense_n*2*V.dense_n);
 			V.column.Allocate((size_t)V.dense_n);
 			V.dense_flag.Allocate(1);
-			V.panel.Allocate((size_t)2*V.dense_n*kPanel+kPanel*kPanel);
-			V.pivots.Allocate(kPanel);
+			V.panel.Allocate((size_t)V.dense_n*kPanel);
+			V.permutation.Allocate((size_t)3*V.dense_n);
 		}
 	}
 	CudaCheck(cudaStreamSynchronize(stream_), "AMG setup");
@@ -726,6 +799,65 @@ template <> float* Amg::ApValues<float>(Level& L)
 {
 	if (L.ap_values32.size() == 0) L.ap_values32.Allocate((size_t)L.ap_blocks*16);
 	return L.ap_values32.get();
+}
+
+// The coarse operator's inverse by the blocked elimination; false when a pivot vanished (or no cluster of
+// the needed size can run here).
+bool Amg::InvertCoarse(Level& Z)
+{
+	const int n = Z.dense_n;
+	const int ctas = (n+kPanelThreads-1)/kPanelThreads;
+	if (ctas > kPanelClusterMax) return false;
+	cudaLaunchConfig_t config = {};
+	config.gridDim = dim3((unsigned)ctas);
+	config.blockDim = dim3(kPanelThreads);
+	config.stream = stream_;
+	cudaLaunchAttribute attribute;
+	attribute.id = cudaLaunchAttributeClusterDimension;
+	attribute.val.clusterDim.x = (unsigned)ctas;
+	attribute.val.clusterDim.y = attribute.val.clusterDim.z = 1;
+	config.attrs = &attribute;
+	config.numAttrs = 1;
+	if (ctas > 8) {
+		CudaCheck(cudaFuncSetAttribute(InversePanelKernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1),
+			"coarse inverse cluster");
+		int clusters = 0;
+		if (cudaOccupancyMaxActiveClusters(&clusters, InversePanelKernel, &config) != cudaSuccess || clusters < 1) {
+			(void)cudaGetLastError();
+			return false;
+		}
+	}
+	double* from = Z.dense.get();
+	double* to = from+(size_t)n*n;
+	int* source = Z.permutation.get();
+	int* order = source+n;
+	int* order_out = order+n;
+	CudaCheck(cudaMemsetAsync(from, 0, (size_t)n*n*sizeof(double), stream_), "coarse matrix");
+	Z.dense_flag.Zero(stream_);
+	DenseScatterKernel<<<Grid(Z.blocks*16, 256), 256, 0, stream_>>>(Z.view(), Z.values.get(), n, from);
+	IdentityOrderKernel<<<Grid(n, 256), 256, 0, stream_>>>(n, order);
+	LaunchCheck("DenseScatterKernel");
+	launches_ += 2;
+	const dim3 tiles(Grid(n, kUpdateTile), Grid(n, kUpdateTile));
+	for (int k0 = 0; k0 < n; k0 += kPanel) {
+		const int b = std::min(kPanel, n-k0);
+		CudaCheck(cudaLaunchKernelEx(&config, InversePanelKernel, n, k0, b, static_cast<const double*>(from),
+			Z.panel.get(), source, Z.dense_flag.get()), "InversePanelKernel");
+		InverseUpdateKernel<<<tiles, 256, 0, stream_>>>(n, k0, b, from, to, Z.panel.get(), source, order, order_out);
+		LaunchCheck("InverseUpdateKernel");
+		std::swap(from, to);
+		std::swap(order, order_out);
+		launches_ += 2;
+	}
+	InverseColumnsKernel<<<Grid((long long)n*n, 256), 256, 0, stream_>>>(n, from, order, to);
+	LaunchCheck("InverseColumnsKernel");
+	launches_ += 1;
+	Z.dense_inverse = to;
+	Z.dense_ld = n;
+	int flag = 0;
+	Z.dense_flag.Download(&flag, 1, stream_);
+	CudaCheck(cudaStreamSynchronize(stream_), "AMG coarse inverse");
+	return flag == 0;
 }
 
 template <class T>
@@ -793,31 +925,14 @@ void Amg::Refresh(const T* values, bool coarse)
 	Level& Z = *levels_.back();
 	if (Z.dense_n == 0 || !coarse) return;
 	coarse_ready_ = true;
-	Z.dense.Zero(stream_);
-	Z.dense_flag.Zero(stream_);
-	DenseScatterKernel<<<Grid(Z.blocks*16, 256), 256, 0, stream_>>>(Z.view(), Z.values.get(), Z.dense_n, Z.dense.get());
-	LaunchCheck("DenseScatterKernel");
 	const int dn = Z.dense_n;
-	AugmentIdentityKernel<<<Grid((long long)dn*dn, 256), 256, 0, stream_>>>(dn, Z.dense.get());
-	LaunchCheck("AugmentIdentityKernel");
-	launches_ += 2;
-	for (int k0 = 0; k0 < dn; k0 += kPanel) {
-		const int b = std::min(kPanel, dn-k0);
-		GaussJordanPanelKernel<<<1, kPanelThreads, 0, stream_>>>(dn, k0, b, Z.dense.get(), Z.panel.get(),
-			Z.pivots.get(), Z.dense_flag.get());
-		GaussJordanUpdateKernel<<<Grid(2LL*dn, kUpdateColumns), 256, 0, stream_>>>(dn, k0, b, Z.dense.get(),
-			Z.panel.get(), Z.pivots.get());
-		launches_ += 2;
-	}
-	LaunchCheck("GaussJordanUpdateKernel");
+	if (InvertCoarse(Z)) return;
 	// a vanishing panel pivot: redo the inverse one column at a time (that path decouples the unknown)
-	int flag = 0;
-	Z.dense_flag.Download(&flag, 1, stream_);
-	CudaCheck(cudaStreamSynchronize(stream_), "AMG coarse inverse");
-	if (flag == 0) return;
 	Z.dense.Zero(stream_);
 	Z.dense_flag.Zero(stream_);
-	DenseScatterKernel<<<Grid(Z.blocks*16, 256), 256, 0, stream_>>>(Z.view(), Z.values.get(), Z.dense_n, Z.dense.get());
+	Z.dense_inverse = Z.dense.get()+dn;
+	Z.dense_ld = 2LL*dn;
+	DenseScatterKernel<<<Grid(Z.blocks*16, 256), 256, 0, stream_>>>(Z.view(), Z.values.get(), 2LL*dn, Z.dense.get());
 	AugmentIdentityKernel<<<Grid((long long)dn*dn, 256), 256, 0, stream_>>>(dn, Z.dense.get());
 	for (int k = 0; k < dn; ++k) {
 		GaussJordanPivotKernel<<<1, 1024, 0, stream_>>>(dn, k, Z.dense.get(), Z.column.get(), Z.dense_flag.get());
@@ -841,7 +956,8 @@ void Amg::Cycle(int l, const T* A, const double* b, double* x, const int* stop, 
 	RestrictKernel<<<C.nodes, 128, 0, stream_>>>(C.nodes, L.agg_order.get(), L.agg_offsets.get(),
 		L.mask.get(), b, C.b.get(), stop, masked ? aggregate_segment_dev_.get() : nullptr, masked ? seg_stop : nullptr);
 	LaunchCheck("RestrictKernel");
-	DenseApplyKernel<<<Grid(C.dense_n, 8), 256, 0, stream_>>>(C.dense_n, C.dense.get(), C.b.get(), C.x.get(), stop);
+	DenseApplyKernel<<<Grid(C.dense_n, 8), 256, 0, stream_>>>(C.dense_n, C.dense_inverse, C.dense_ld, C.b.get(),
+		C.x.get(), stop);
 	LaunchCheck("DenseApplyKernel");
 	(void)A;      // the fine operator enters through A P, refreshed with it
 	CoarseCorrectionKernel<T><<<Grid(4LL*L.nodes, 256), 256, 0, stream_>>>(L.nodes, L.agg.get(), L.mask.get(),
@@ -873,8 +989,8 @@ AmgResidentView Amg::ResidentView()
 	v.agg_order = L.agg_order.get();
 	v.agg_offsets = L.agg_offsets.get();
 	v.mask = L.mask.get();
-	v.dense = C.dense.get()+C.dense_n;
-	v.dense_ld = 2LL*C.dense_n;
+	v.dense = C.dense_inverse;
+	v.dense_ld = C.dense_ld;
 	v.coarse_rhs = C.b.get();
 	v.coarse_x = C.x.get();
 	v.ap_rows = L.ap_rows.get();

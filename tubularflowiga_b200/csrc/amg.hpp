@@ -84,6 +84,7 @@ private:
 	bool segment_maps_ = false;
 	template <class T> T* ApValues(Level& level);   // A P blocks in the fine matrix's precision
 	void BuildFromStrength(std::vector<double> s);
+	bool InvertCoarse(Level& coarse);
 	std::vector<std::unique_ptr<Level>> levels_;
 	DevicePatternView fine_;
 	std::vector<int32_t> fine_rows_, fine_columns_;

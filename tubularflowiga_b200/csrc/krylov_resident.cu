@@ -760,6 +760,9 @@ void ResidentKrylov::Plan(const DevicePatternView& pattern, const AmgResidentVie
 	CudaCheck(cudaDeviceGetAttribute(&cooperative, cudaDevAttrCooperativeLaunch, device), "device attribute");
 	CudaCheck(cudaDeviceGetAttribute(&shared_max, cudaDevAttrMaxSharedMemoryPerBlockOptin, device), "device attribute");
 	if (!cooperative) return;
+	const Kernel kernel = KernelOf(kind_);
+	cudaFuncAttributes attributes;
+	CudaCheck(cudaFuncGetAttributes(&attributes, reinterpret_cast<const void*>(kernel)), "resident GMRES attributes");
 	// the slice of an average CTA alone already says whether large systems fit
 	const size_t entry = kind_ == kFlexFloat ? 4 : 8;
 	if ((size_t)fields*pattern.nodes/sms*(restart_+1)*entry > (size_t)shared_max) return;
@@ -772,10 +775,12 @@ void ResidentKrylov::Plan(const DevicePatternView& pattern, const AmgResidentVie
 	else for (const int64_t e : segments_) bounds.push_back((int32_t)(e/fields));
 	groups_ = (int)bounds.size()-1;
 	if (groups_ > sms) return;
-	// one CTA per SM, fewer where a CTA would get less than about 100 KB of the matrix; CTAs over the groups
-	// by blocks, at least one each
+	// one CTA per SM, fewer where a CTA would get less than about 100 KB of the matrix and 60 KB of basis; CTAs
+	// over the groups by blocks, at least one each
 	const long long blocks = rows[pattern.nodes];
-	ctas_ = (int)std::min<long long>(sms, std::max<long long>({1, groups_, blocks/(fields == 4 ? 1024 : 4096)}));
+	const long long basis = (long long)fields*pattern.nodes*(restart_+1)*(long long)entry;
+	ctas_ = (int)std::min<long long>(sms, std::max<long long>({1, groups_, blocks/(fields == 4 ? 1024 : 4096),
+		basis/60000}));
 	std::vector<int> share(groups_, 1);
 	for (int left = ctas_-groups_; left > 0; --left) {
 		int best = 0;
@@ -811,9 +816,6 @@ void ResidentKrylov::Plan(const DevicePatternView& pattern, const AmgResidentVie
 	if (fields == 2) pieces_ = 1;
 	const size_t m1 = (size_t)restart_+1;
 	smem_ = ((size_t)slice_*(1+pieces_)+kThreads+8*m1+(m1 & 1))*sizeof(double)+m1*slice_*entry;
-	const Kernel kernel = KernelOf(kind_);
-	cudaFuncAttributes attributes;
-	CudaCheck(cudaFuncGetAttributes(&attributes, reinterpret_cast<const void*>(kernel)), "resident GMRES attributes");
 	if (smem_+attributes.sharedSizeBytes > (size_t)shared_max) return;
 	if (amg) {
 		if (4*(long long)amg->coarse > (long long)ctas_*kDenseRows) return;
