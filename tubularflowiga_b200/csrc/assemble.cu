@@ -7,188 +7,191 @@
 // tangent is the exact derivative (NavierStokesElement.hpp:244-312), not the
 // frozen-tau tangent of the reference GPU kernel (IgaCudaKernels.cuh:380-396).
 //
-// Organisation.  At each quadrature point q every term of the tangent is a
-// product (test feature s of N_a) x (trial feature t of N_b) with
-// s in {N, dN/dx, dN/dy, dN/dz} and t in {N, dN/dx, dN/dy, dN/dz, Lap N}, so
-//   K^{if}_{ab} = sum_q sum_s Psi_s(a,q) * G^{if}_s(b,q),
-//   G^{if}_s(b,q) = measure_q * sum_t M_q^{if}[s][t] Phi_t(b,q),
-// a GEMM of K = 64 points x 4 test features.  One CTA owns one element and one
-// row field i; it builds the 4x5 coefficient matrices M_q^{i f} once per point,
-// forms G in shared memory chunk by chunk and accumulates the 64 x 256 block
-// (a, (b, f)) in registers with an 8x8 FP64 tile per thread, then adds the
-// result into block CSR through the precomputed element -> block map.
+// Organisation.  Every term of the tangent is a product (test feature s of N_a) x (G_s of N_b) at a point
+// (vms_tangent.cuh), so per row field i it is a matrix product over k = (point, s),
+//   K^{if}_{ab} = sum_k G^{if}[(b, f)][k] Psi[k][a],   K = 64 points x 4 test features,
+// and runs on the FP64 tensor path (mma.sync m16n8k16: operands in registers, so that shared memory serves
+// three words per 64 products instead of one).  A CTA of 256 threads owns (element, row field, half of the
+// functions b): 128 rows (b, f) x 64 functions a in registers, two CTAs per SM, so that one builds G while the
+// other multiplies.  Per chunk of four points: G and Psi into padded shared buffers (two of each, one barrier a
+// chunk), then one m16n8k16 per eight functions a.  Rows, columns and CTAs past the element's own function
+// count are skipped: elements at patch boundaries have 18 to 48 functions, and on the benchmark's meshes
+// nen^2 is 40 to 65 % of 64^2.  The FP64 pipe bounds it.  The kernel it replaces (one CTA per SM, 8 x 8
+// register tiles of scalar products over all 64 x 256 entries, the point state recomputed for each row
+// field) took 34.5 ms for the 12,800-element section and 3.4 ms for the 1,280-element cylinder.
 #include "common.hpp"
 #include "kernels.cuh"
-#include "l2_prefetch.cuh"
 #include "vms_point.cuh"
+#include "vms_tangent.cuh"
 
 namespace tfiga {
 namespace {
 
 constexpr int kThreads = 256;
-constexpr int kChunkPoints = 8;                 // quadrature points per GEMM chunk
-constexpr int kChunkK = kChunkPoints*4;         // GEMM depth per chunk
-template <int NP>
-__global__ void __launch_bounds__(kThreads, 1) AssembleKernel(DeviceMeshView mesh, const double* __restrict__ phi,
-	const double* __restrict__ qdata, const int32_t* __restrict__ element_blocks, const double* __restrict__ state,
-	const double* __restrict__ previous, AssemblyParams prm, double* __restrict__ values, double* __restrict__ rhs)
+constexpr int kChunkPoints = 4;                 // points per chunk
+constexpr int kChunkK = kChunkPoints*4;         // depth of a chunk
+constexpr int kHalf = 32;                       // functions b per CTA at most
+// Row strides (in doubles) that keep fragment loads free of bank conflicts: 16 lanes read 4 rows x 4
+// columns of G and 4 x 4 of Psi.
+constexpr int kGStride = kChunkK+4;
+constexpr int kPsiStride = kMaxBasis+4;
+
+struct AssembleShared {
+	double G[2][4*kHalf][kGStride];
+	double Psi[2][kChunkK][kPsiStride];
+	double pack[2][kChunkPoints][kPack];
+};
+
+__device__ __forceinline__ void Mma16816(double c[4], const double a[8], const double b[4])
 {
-	static_assert(NP == 64, "the register tiling assumes 64 padded basis functions");
-	extern __shared__ __align__(16) double sm[];
-	double* U = sm;                          // [NP][4] current state
-	double* Up = U+NP*4;                     // [NP][4] previous velocity
-	double* QS = Up+NP*4;                    // [64][kQS]
-	double* Msm = QS+kQuad*kQS;              // [64][kCoef]
-	double* RC = Msm+kQuad*kCoef;            // [64][4]
-	double* Psi = RC+kQuad*4;                // [kChunkK][NP]
-	double* Gs = Psi+kChunkK*NP;             // [kChunkK][4*NP]
+	asm volatile("mma.sync.aligned.m16n8k16.row.col.f64.f64.f64.f64 {%0, %1, %2, %3}, {%4, %5, %6, %7, %8, %9, %10, %11}, "
+		"{%12, %13, %14, %15}, {%0, %1, %2, %3};"
+		: "+d"(c[0]), "+d"(c[1]), "+d"(c[2]), "+d"(c[3])
+		: "d"(a[0]), "d"(a[1]), "d"(a[2]), "d"(a[3]), "d"(a[4]), "d"(a[5]), "d"(a[6]), "d"(a[7]), "d"(b[0]), "d"(b[1]),
+		"d"(b[2]), "d"(b[3]));
+}
 
-	const int e = blockIdx.x >> 2;
-	const int row = blockIdx.x & 3;
-	const int tid = threadIdx.x;
-	const int warp = tid >> 5, lane = tid & 31;
-	const int begin = mesh.element_offsets[e];
-	const int nen = mesh.element_offsets[e+1]-begin;
-	const double* P = phi+(size_t)e*kFeatures*kQuad*NP;
-	if (tid == 0) PrefetchL2(P, kFeatures*kQuad*NP*8);
-
-	// 1. Gather nodal state.
-	for (int a = tid; a < NP; a += kThreads) {
-		double s0 = 0.0, s1 = 0.0, s2 = 0.0, s3 = 0.0, p0 = 0.0, p1 = 0.0, p2 = 0.0;
-		if (a < nen) {
-			const size_t node = (size_t)mesh.connectivity[begin+a];
-			const double2 x01 = *reinterpret_cast<const double2*>(state+4*node);
-			const double2 x23 = *reinterpret_cast<const double2*>(state+4*node+2);
-			s0 = x01.x; s1 = x01.y; s2 = x23.x; s3 = x23.y;
-			if (prm.dt > 0.0) {
-				const double2 y01 = *reinterpret_cast<const double2*>(previous+4*node);
-				p0 = y01.x; p1 = y01.y; p2 = previous[4*node+2];
+template <int I>
+__device__ __forceinline__ void AssembleRow(AssembleShared& sm, const double* __restrict__ P,
+	const double* __restrict__ packs, const int32_t* __restrict__ EB, int nen, int b0, int bn, double irho, double nu,
+	double* __restrict__ values)
+{
+	const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+	const int columns = (nen+7) & ~7;            // functions a in steps of eight
+	// builder: a warp per (column-field pair, point), a lane per function b
+	const int pair = warp >> 2, point = warp & 3;
+	const bool builds = lane < bn;
+	double ph[kFeatures];
+	auto load = [&](int c) {
+		if (builds) {
+			const double* p = P+(size_t)(c*kChunkPoints+point)*kMaxBasis+b0+lane;
+			#pragma unroll
+			for (int t = 0; t < kFeatures; ++t) ph[t] = __ldg(p+(size_t)t*kQuad*kMaxBasis);
+		}
+	};
+	auto stage = [&](int c, int buffer) {
+		// Psi rows k = 4 point + s, sixteen rows of up to 32 16-byte units, two rows per warp; the numbers
+		#pragma unroll
+		for (int r = 0; r < 2; ++r) {
+			const int k = 2*warp+r;
+			if (2*lane < columns) {
+				const uint32_t dst = (uint32_t)__cvta_generic_to_shared(&sm.Psi[buffer][k][2*lane]);
+				const double* src = P+((size_t)(k & 3)*kQuad+c*kChunkPoints+(k >> 2))*kMaxBasis+2*lane;
+				asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" :: "r"(dst), "l"(src) : "memory");
 			}
 		}
-		U[a*4] = s0; U[a*4+1] = s1; U[a*4+2] = s2; U[a*4+3] = s3;
-		Up[a*4] = p0; Up[a*4+1] = p1; Up[a*4+2] = p2; Up[a*4+3] = 0.0;
-	}
-	__syncthreads();
-
-	// 2. State at every point: a warp per point, lanes over basis functions.
-	for (int q = warp; q < kQuad; q += kThreads/32) {
-		double v[22];
-		#pragma unroll
-		for (int k = 0; k < 22; ++k) v[k] = 0.0;
-		for (int a = lane; a < NP; a += 32) {
-			const double n = P[(0*kQuad+q)*NP+a];
-			const double g0 = P[(1*kQuad+q)*NP+a], g1 = P[(2*kQuad+q)*NP+a], g2 = P[(3*kQuad+q)*NP+a];
-			const double l = P[(4*kQuad+q)*NP+a];
-			const double u0 = U[a*4], u1 = U[a*4+1], u2 = U[a*4+2], u3 = U[a*4+3];
-			v[0] += n*u0; v[1] += n*u1; v[2] += n*u2; v[3] += n*u3;
-			v[4] += n*Up[a*4]; v[5] += n*Up[a*4+1]; v[6] += n*Up[a*4+2];
-			const double uf[4] = {u0, u1, u2, u3};
-			#pragma unroll
-			for (int f = 0; f < 4; ++f) { v[7+3*f] += g0*uf[f]; v[8+3*f] += g1*uf[f]; v[9+3*f] += g2*uf[f]; }
-			v[19] += l*u0; v[20] += l*u1; v[21] += l*u2;
+		if (tid < kChunkPoints*kPack/2) {
+			const uint32_t dst = (uint32_t)__cvta_generic_to_shared(&sm.pack[buffer][0][0]+2*tid);
+			asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" :: "r"(dst),
+				"l"(packs+(size_t)c*kChunkPoints*kPack+2*tid) : "memory");
 		}
-		#pragma unroll
-		for (int k = 0; k < 22; ++k)
-			#pragma unroll
-			for (int o = 16; o > 0; o >>= 1) v[k] += __shfl_xor_sync(0xffffffffu, v[k], o);
-		if (lane == 0)
-			#pragma unroll
-			for (int k = 0; k < 22; ++k) QS[q*kQS+k] = v[k];
-	}
-	__syncthreads();
-
-	// 3. Coefficients of this CTA's row field at every point.
-	if (tid < kQuad) {
-		PointState S;
-		const double* s = QS+tid*kQS;
-		for (int c = 0; c < 3; ++c) {
-			S.u[c] = s[kU+c]; S.up[c] = s[kUp+c]; S.lap[c] = s[kLap+c]; S.gp[c] = s[kGrad+9+c];
-			for (int d = 0; d < 3; ++d) S.gv[c][d] = s[kGrad+3*c+d];
+		asm volatile("cp.async.commit_group;" ::: "memory");
+	};
+	auto build = [&](int buffer) {
+		if (!builds) return;
+		const double* pk = sm.pack[buffer][point];
+		const auto coef = [&](int k) { return pk[k]; };
+		const double n = ph[0], g[3] = {ph[1], ph[2], ph[3]};
+		const double l = pk[kPackU]*g[0]+pk[kPackU+1]*g[1]+pk[kPackU+2]*g[2]-nu*ph[4];
+		auto put = [&](int f, const double v[4]) {
+			double2* d = reinterpret_cast<double2*>(&sm.G[buffer][4*lane+f][4*point]);
+			d[0] = make_double2(v[0], v[1]);
+			d[1] = make_double2(v[2], v[3]);
+		};
+		double v[4];
+		if (pair == 0) {
+			TangentColumn<I, 0>(coef, n, g, l, irho, v);
+			put(0, v);
+			TangentColumn<I, 1>(coef, n, g, l, irho, v);
+			put(1, v);
+		} else {
+			TangentColumn<I, 2>(coef, n, g, l, irho, v);
+			put(2, v);
+			TangentColumn<I, 3>(coef, n, g, l, irho, v);
+			put(3, v);
 		}
-		S.p = s[kP];
-		RowCoefficients(row, S, qdata+((size_t)e*kQuad+tid)*kQData, prm, Msm+tid*kCoef, RC+tid*4);
-	}
-	__syncthreads();
-
-	// 4. Residual of row field `row` (rhs holds -r).
-	if (rhs != nullptr && tid < nen) {
-		double r = 0.0;
-		for (int q = 0; q < kQuad; ++q)
-			#pragma unroll
-			for (int s = 0; s < 4; ++s) r += P[(s*kQuad+q)*NP+tid]*RC[q*4+s];
-		atomicAdd(rhs+4*(size_t)mesh.connectivity[begin+tid]+row, r);
-	}
-	if (values == nullptr) return;
-
-	// 5. Tangent: acc[a-tile][col-tile] over K = 64 points x 4 test features.
-	double acc[8][8];
+	};
+	constexpr int kTiles = kMaxBasis/8;
+	double acc[kTiles][4];
 	#pragma unroll
-	for (int i = 0; i < 8; ++i)
+	for (int t = 0; t < kTiles; ++t)
 		#pragma unroll
-		for (int j = 0; j < 8; ++j) acc[i][j] = 0.0;
-	const int ta = warp, tb = lane;
-	for (int qc = 0; qc < kQuad; qc += kChunkPoints) {
-		for (int idx = tid; idx < kChunkK*NP; idx += kThreads) {
-			const int k = idx/NP, a = idx%NP;
-			Psi[idx] = P[((k&3)*kQuad+qc+(k>>2))*NP+a];
-		}
-		{
-			const int c = tid, b = c >> 2, f = c & 3;   // column (b, f) of G
-			#pragma unroll 2
-			for (int qq = 0; qq < kChunkPoints; ++qq) {
-				const int q = qc+qq;
-				double ph[5];
-				#pragma unroll
-				for (int t = 0; t < 5; ++t) ph[t] = P[(t*kQuad+q)*NP+b];
-				const double* Mq = Msm+q*kCoef+f*20;
-				#pragma unroll
-				for (int s = 0; s < 4; ++s)
-					Gs[(qq*4+s)*(4*NP)+c] = Mq[s*5]*ph[0]+Mq[s*5+1]*ph[1]+Mq[s*5+2]*ph[2]+Mq[s*5+3]*ph[3]
-						+Mq[s*5+4]*ph[4];
+		for (int k = 0; k < 4; ++k) acc[t][k] = 0.0;
+	const int gr = lane >> 2, t4 = lane & 3;
+	const bool multiplies = 4*warp < bn;         // this warp's sixteen rows: functions 4 warp .. 4 warp + 3
+	constexpr int kChunks = kQuad/kChunkPoints;
+	load(0);
+	stage(0, 0);
+	asm volatile("cp.async.wait_group 0;" ::: "memory");
+	__syncthreads();
+	build(0);
+	load(1);
+	stage(1, 1);
+	for (int c = 0; c < kChunks; ++c) {
+		const int buffer = c & 1;
+		asm volatile("cp.async.wait_group 0;" ::: "memory");
+		__syncthreads();                         // G and Psi of chunk c, numbers and Psi of chunk c + 1
+		if (c+1 < kChunks) build(buffer^1);
+		if (c+2 < kChunks) load(c+2);
+		if (multiplies) {
+			double a[8];
+			#pragma unroll
+			for (int j = 0; j < 4; ++j) {
+				a[2*j] = sm.G[buffer][16*warp+gr][4*j+t4];
+				a[2*j+1] = sm.G[buffer][16*warp+gr+8][4*j+t4];
 			}
-		}
-		__syncthreads();
-		#pragma unroll 2
-		for (int k = 0; k < kChunkK; ++k) {
-			const double2* pr = reinterpret_cast<const double2*>(Psi+k*NP+ta*8);
-			const double2 p0 = pr[0], p1 = pr[1], p2 = pr[2], p3 = pr[3];
-			const double* gr = Gs+k*(4*NP)+2*tb;
-			const double2 g0 = *reinterpret_cast<const double2*>(gr);
-			const double2 g1 = *reinterpret_cast<const double2*>(gr+64);
-			const double2 g2 = *reinterpret_cast<const double2*>(gr+128);
-			const double2 g3 = *reinterpret_cast<const double2*>(gr+192);
-			const double pa[8] = {p0.x, p0.y, p1.x, p1.y, p2.x, p2.y, p3.x, p3.y};
-			const double gb[8] = {g0.x, g0.y, g1.x, g1.y, g2.x, g2.y, g3.x, g3.y};
 			#pragma unroll
-			for (int i = 0; i < 8; ++i)
-				#pragma unroll
-				for (int j = 0; j < 8; ++j) acc[i][j] = fma(pa[i], gb[j], acc[i][j]);
+			for (int t = 0; t < kTiles; ++t)
+				if (8*t < columns) {
+					double b[4];
+					#pragma unroll
+					for (int j = 0; j < 4; ++j) b[j] = sm.Psi[buffer][4*j+t4][8*t+gr];
+					Mma16816(acc[t], a, b);
+				}
 		}
-		__syncthreads();
+		__syncthreads();                         // chunk c's buffers are free
+		if (c+2 < kChunks) stage(c+2, buffer);
 	}
-
-	// 6. Scatter-add into block CSR: column 2*tb + 64*j + s is (b = 16j + tb/2, f = 2(tb&1) + s).
-	const int32_t* EB = element_blocks+(size_t)e*NP*NP;
-	const int f0 = 2*(tb & 1);
+	// rows gr and gr + 8 are (function 4 warp + gr / 4 [+ 2], field gr % 4), columns 8 t + 2 t4 [+ 1] functions a:
+	// four lanes add one block row of a block, 32 contiguous bytes
+	if (!multiplies) return;
 	#pragma unroll
-	for (int i = 0; i < 8; ++i) {
-		const int a = ta*8+i;
-		if (a >= nen) continue;
+	for (int h = 0; h < 2; ++h) {
+		const int bl = 4*warp+(gr >> 2)+2*h;
+		if (bl >= bn) continue;
+		const int b = b0+bl;
 		#pragma unroll
-		for (int j = 0; j < 4; ++j) {
-			const int b = 16*j+(tb >> 1);
-			const int block = b < nen ? EB[a*NP+b] : -1;
-			if (block < 0) continue;
-			double* dst = values+(size_t)block*16+row*4+f0;
-			atomicAdd(dst, acc[i][2*j]);
-			atomicAdd(dst+1, acc[i][2*j+1]);
+		for (int t = 0; t < kTiles; ++t) {
+			#pragma unroll
+			for (int k = 0; k < 2; ++k) {
+				const int a = 8*t+2*t4+k;
+				const int block = a < nen ? EB[a*kMaxBasis+b] : -1;
+				if (block >= 0) atomicAdd(values+(size_t)block*16+I*4+(gr & 3), acc[t][2*h+k]);
+			}
 		}
 	}
 }
 
-constexpr size_t SharedBytes(int np)
+__global__ void __launch_bounds__(kThreads, 2) AssembleKernel(DeviceMeshView mesh, int first,
+	const double* __restrict__ phi, const double* __restrict__ packs, const int32_t* __restrict__ element_blocks,
+	double irho, double nu, double* __restrict__ values)
 {
-	return sizeof(double)*(size_t)(np*4+np*4+kQuad*kQS+kQuad*kCoef+kQuad*4+kChunkK*np+kChunkK*4*np);
+	extern __shared__ __align__(16) unsigned char raw[];
+	AssembleShared& sm = *reinterpret_cast<AssembleShared*>(raw);
+	const int local = blockIdx.x >> 3, row = (blockIdx.x >> 1) & 3, half = blockIdx.x & 1;
+	const int e = first+local;
+	const int nen = mesh.element_offsets[e+1]-mesh.element_offsets[e];
+	// the functions b in two even parts of whole warps' rows, one part where 32 hold them all
+	const int part = nen > kHalf ? (nen+7)/8*4 : nen;
+	const int b0 = half*part, bn = min(part, nen-b0);
+	if (bn <= 0) return;
+	const double* P = phi+(size_t)e*kFeatures*kQuad*kMaxBasis;
+	const double* pk = packs+(size_t)local*kQuad*kPack;
+	const int32_t* EB = element_blocks+(size_t)e*kMaxBasis*kMaxBasis;
+	if (row == 0) AssembleRow<0>(sm, P, pk, EB, nen, b0, bn, irho, nu, values);
+	else if (row == 1) AssembleRow<1>(sm, P, pk, EB, nen, b0, bn, irho, nu, values);
+	else if (row == 2) AssembleRow<2>(sm, P, pk, EB, nen, b0, bn, irho, nu, values);
+	else AssembleRow<3>(sm, P, pk, EB, nen, b0, bn, irho, nu, values);
 }
 
 // Elements with 65..80 basis functions (rare: the spline extraction's extraordinary vertices), from
@@ -328,22 +331,15 @@ __global__ void __launch_bounds__(kLargeThreads) AssembleLargeKernel(DeviceMeshV
 
 } // namespace
 
-void LaunchAssemble(const DeviceMeshView& mesh, const double* phi, const double* qdata,
-	const int32_t* element_blocks, const double* state, const double* previous, AssemblyParams params,
-	double* values, double* rhs, cudaStream_t stream)
+void LaunchAssembleTangent(const DeviceMeshView& mesh, int first, int count, const double* phi, const double* packs,
+	const int32_t* element_blocks, AssemblyParams params, double* values, cudaStream_t stream)
 {
-	if (mesh.elements == 0) return;
-	constexpr size_t bytes = SharedBytes(kMaxBasis);
-	static bool configured = false;
-	if (!configured) {
-		CudaCheck(cudaFuncSetAttribute(AssembleKernel<kMaxBasis>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-			(int)bytes), "assembly shared-memory attribute");
-		configured = true;
-	}
-	const long long ctas = 4LL*mesh.elements;
-	if (ctas > 0x7fffffffLL) Fail(-7, "too many elements for one assembly launch");
-	AssembleKernel<kMaxBasis><<<(unsigned)ctas, kThreads, bytes, stream>>>(mesh, phi, qdata, element_blocks,
-		state, previous, params, values, rhs);
+	if (count == 0) return;
+	if (8LL*count > 0x7fffffffLL) Fail(-7, "too many elements for one assembly launch");
+	CudaCheck(cudaFuncSetAttribute(AssembleKernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+		(int)sizeof(AssembleShared)), "assembly shared-memory attribute");
+	AssembleKernel<<<8u*(unsigned)count, kThreads, sizeof(AssembleShared), stream>>>(mesh, first, phi, packs,
+		element_blocks, 1.0/params.density, params.viscosity/params.density, values);
 	LaunchCheck("AssembleKernel");
 }
 

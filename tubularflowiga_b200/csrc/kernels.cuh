@@ -17,6 +17,7 @@ namespace tfiga {
 constexpr int kQuad = 64;       // 4x4x4 Gauss points
 constexpr int kFeatures = 5;    // N, dN/dx, dN/dy, dN/dz, Laplacian
 constexpr int kQData = 10;
+constexpr int kPointNumbers = 72;   // numbers of the factored tangent per point (vms_tangent.cuh)
 constexpr int kMaxBasis = 64;   // padded basis count NP of the device tables
 // Elements with 65..80 basis functions (the reference's limit, solvers/cuda/include/DeviceMesh.hpp:55-56)
 // keep their own tables padded to 80 and go through the large-element kernels.
@@ -62,12 +63,19 @@ void LaunchElementBlocksLarge(const DeviceMeshView& mesh, const DevicePatternVie
 void LaunchFaceCoefficients(const DeviceMeshView& mesh, int faces, const int32_t* face_element,
 	const int32_t* face_index, double* face_coef, int stride, cudaStream_t stream);
 
+// ---- point_stream.cu ----------------------------------------------------
+// The elements [first, first + count): the tangent's numbers of every point (vms_tangent.cuh) into packs64
+// ([element - first][point][72]) or packs32 ([element - first][point pair][72][2]) (at most one given), and
+// the FP64 residual ADDED into rhs (= -r; may be null).
+void LaunchPointStream(const DeviceMeshView& mesh, int first, int count, const double* phi, const double* qdata,
+	const double* state, const double* previous, AssemblyParams params, double* packs64, float* packs32, double* rhs,
+	cudaStream_t stream);
+
 // ---- assemble.cu --------------------------------------------------------
-// Exact-tangent VMS assembly: jacobian values (may be null: residual only) and
-// rhs (= -r) are ADDED to.
-void LaunchAssemble(const DeviceMeshView& mesh, const double* phi, const double* qdata,
-	const int32_t* element_blocks, const double* state, const double* previous, AssemblyParams params,
-	double* values, double* rhs, cudaStream_t stream);
+// Exact FP64 VMS tangent of the elements [first, first + count), from the points' numbers `packs`
+// (LaunchPointStream's packs64), ADDED into values.
+void LaunchAssembleTangent(const DeviceMeshView& mesh, int first, int count, const double* phi, const double* packs,
+	const int32_t* element_blocks, AssemblyParams params, double* values, cudaStream_t stream);
 // The same element (FP64 point state, coefficients, residual and exact tangent) for the elements
 // [first, first + count) with up to 80 basis functions, from their 80-wide tables; values (FP64 or
 // FP32 storage, may be null: residual only) and rhs (may be null: tangent only) are ADDED to.

@@ -338,14 +338,32 @@ void NsSolver::AssembleResidual()
 	rhs_.Zero(stream_);
 	profiler_.End(stream_);
 	profiler_.Begin(Profiler::kResidual, stream_);
-	LaunchTangentPoint(mesh_.regular_view(), mesh_.phi(), mesh_.qdata(), state_.get(), previous_.get(),
-		{params_.density, params_.viscosity, params_.dt}, nullptr, nullptr, rhs_.get(), stream_);
+	LaunchPointStream(mesh_.regular_view(), 0, (int)mesh_.regular_elements(), mesh_.phi(), mesh_.qdata(), state_.get(),
+		previous_.get(), {params_.density, params_.viscosity, params_.dt}, nullptr, nullptr, rhs_.get(), stream_);
 	LargeElements<double>(nullptr, rhs_.get());
 	profiler_.End(stream_);
 	profiler_.Begin(Profiler::kVector, stream_);
 	LaunchAxpy(n4_, 1.0, traction_.get(), rhs_.get(), stream_);
 	profiler_.End(stream_);
 	launches_ += 2;
+}
+
+void NsSolver::AssembleFp64(double* rhs)
+{
+	// in slabs of elements, whose points' numbers (36 KiB per element) share one workspace
+	constexpr int kSlab = 16384;
+	const int count = (int)mesh_.regular_elements();
+	const AssemblyParams prm{params_.density, params_.viscosity, params_.dt};
+	if (packs_.size() == 0) packs_.Allocate((size_t)std::min(kSlab, count)*kQuad*kPointNumbers);
+	values_.Zero(stream_);
+	for (int first = 0; first < count; first += kSlab) {
+		const int slab = std::min(kSlab, count-first);
+		LaunchPointStream(mesh_.regular_view(), first, slab, mesh_.phi(), mesh_.qdata(), state_.get(), previous_.get(), prm,
+			packs_.get(), nullptr, rhs, stream_);
+		LaunchAssembleTangent(mesh_.regular_view(), first, slab, mesh_.phi(), packs_.get(), mesh_.element_blocks(), prm,
+			values_.get(), stream_);
+		launches_ += 2;
+	}
 }
 
 void NsSolver::AssembleTangent()
@@ -356,9 +374,7 @@ void NsSolver::AssembleTangent()
 	}
 	amg_current_ = false;
 	profiler_.Begin(Profiler::kAssembly, stream_);
-	values_.Zero(stream_);
-	LaunchAssemble(mesh_.regular_view(), mesh_.phi(), mesh_.qdata(), mesh_.element_blocks(), state_.get(),
-		previous_.get(), {params_.density, params_.viscosity, params_.dt}, values_.get(), nullptr, stream_);
+	AssembleFp64(nullptr);
 	LargeElements<double>(values_.get(), nullptr);
 	if (mixed()) {
 		LaunchToFloat((long long)blocks()*16, values_.get(), values32_.get(), stream_);
@@ -380,11 +396,9 @@ void NsSolver::Assemble()
 		return;
 	}
 	amg_current_ = false;
-	values_.Zero(stream_);
 	rhs_.Zero(stream_);
 	profiler_.Begin(Profiler::kAssembly, stream_);
-	LaunchAssemble(mesh_.regular_view(), mesh_.phi(), mesh_.qdata(), mesh_.element_blocks(), state_.get(),
-		previous_.get(), {params_.density, params_.viscosity, params_.dt}, values_.get(), rhs_.get(), stream_);
+	AssembleFp64(rhs_.get());
 	LargeElements<double>(values_.get(), rhs_.get());
 	profiler_.End(stream_);
 	LaunchAxpy(n4_, 1.0, traction_.get(), rhs_.get(), stream_);

@@ -125,6 +125,8 @@ private:
 	// tensor-core contraction; builds the AMG on first use).
 	void AssembleResidual();
 	void AssembleTangent();
+	// FP64 tangent into values_ (cleared first) and, when rhs is given, the residual added into it.
+	void AssembleFp64(double* rhs);
 	// The elements with 65..80 basis functions (FP64 large-element kernel): tangent added into values
 	// and residual into rhs, either may be null.  No launch when the mesh has none.
 	template <class T> void LargeElements(T* values, double* rhs);
@@ -152,6 +154,7 @@ private:
 	DeviceArray<double> values_, rhs_, state_, previous_, update_, traction_, velocity_bc_, pressure_bc_;
 	DeviceArray<float> values32_;
 	DeviceArray<float> coef32_;              // tensor-core tangent: point coefficients [e][4][80][64]
+	DeviceArray<double> packs_;              // FP64 tangent: the points' numbers of a slab of elements
 	DeviceArray<double> point_state_;        // fused tensor-core tangent: FP64 point state [e][64][22]
 	int tangent_kernel_ = 0;                 // TFIGA_TANGENT_* in use
 	double tune_ms_[3] = {0.0, 0.0, 0.0};    // autotuner: coefficient-array (pair), fused, element times
