@@ -10,15 +10,17 @@
 // Organisation.  Every term of the tangent is a product (test feature s of N_a) x (G_s of N_b) at a point
 // (vms_tangent.cuh), so per row field i it is a matrix product over k = (point, s),
 //   K^{if}_{ab} = sum_k G^{if}[(b, f)][k] Psi[k][a],   K = 64 points x 4 test features,
-// and runs on the FP64 tensor path (mma.sync m16n8k16: operands in registers, so that shared memory serves
+// and runs on the FP64 tensor path (mma.sync: operands in registers, so that shared memory serves
 // three words per 64 products instead of one).  A CTA of 256 threads owns (element, row field, half of the
 // functions b): 128 rows (b, f) x 64 functions a in registers, two CTAs per SM, so that one builds G while the
-// other multiplies.  Per chunk of four points: G and Psi into padded shared buffers (two of each, one barrier a
-// chunk), then one m16n8k16 per eight functions a.  Rows, columns and CTAs past the element's own function
+// other multiplies.  Per chunk of four points: G and Psi into padded shared buffers (one barrier a chunk), then
+// the product.  m16n8k4 and not k16: scalar FP64 work of the builders queues behind the products on the same
+// pipe, 32 cycles each instead of 128.  Rows, columns and CTAs past the element's own function
 // count are skipped: elements at patch boundaries have 18 to 48 functions, and on the benchmark's meshes
 // nen^2 is 40 to 65 % of 64^2.  The FP64 pipe bounds it.  The kernel it replaces (one CTA per SM, 8 x 8
 // register tiles of scalar products over all 64 x 256 entries, the point state recomputed for each row
-// field) took 34.5 ms for the 12,800-element section and 3.4 ms for the 1,280-element cylinder.
+// field) took 34.5 ms for the 12,800-element section and 3.4 ms for the 1,280-element cylinder; this one takes
+// 12.6 and 0.88 ms, 63 % of the FP64 pipe's time at 64 products per cycle and SM.
 #include "common.hpp"
 #include "kernels.cuh"
 #include "vms_point.cuh"
@@ -31,24 +33,22 @@ constexpr int kThreads = 256;
 constexpr int kChunkPoints = 4;                 // points per chunk
 constexpr int kChunkK = kChunkPoints*4;         // depth of a chunk
 constexpr int kHalf = 32;                       // functions b per CTA at most
-// Row strides (in doubles) that keep fragment loads free of bank conflicts: 16 lanes read 4 rows x 4
-// columns of G and 4 x 4 of Psi.
+// Strides (in doubles) that keep shared accesses free of bank conflicts: 16 lanes read 4 rows (fields of one
+// function) x 4 columns of G and 4 x 4 of Psi; 8 lanes store 16 bytes each of eight functions.
 constexpr int kGStride = kChunkK+4;
+constexpr int kGFunction = 4*kGStride+2;
 constexpr int kPsiStride = kMaxBasis+4;
 
 struct AssembleShared {
-	double G[2][4*kHalf][kGStride];
-	double Psi[2][kChunkK][kPsiStride];
-	double pack[2][kChunkPoints][kPack];
+	double G[2][kHalf*kGFunction];
+	double Psi[3][kChunkK][kPsiStride];
+	double pack[3][kChunkPoints][kPack];
 };
 
-__device__ __forceinline__ void Mma16816(double c[4], const double a[8], const double b[4])
+__device__ __forceinline__ void Mma1684(double c[4], double a0, double a1, double b)
 {
-	asm volatile("mma.sync.aligned.m16n8k16.row.col.f64.f64.f64.f64 {%0, %1, %2, %3}, {%4, %5, %6, %7, %8, %9, %10, %11}, "
-		"{%12, %13, %14, %15}, {%0, %1, %2, %3};"
-		: "+d"(c[0]), "+d"(c[1]), "+d"(c[2]), "+d"(c[3])
-		: "d"(a[0]), "d"(a[1]), "d"(a[2]), "d"(a[3]), "d"(a[4]), "d"(a[5]), "d"(a[6]), "d"(a[7]), "d"(b[0]), "d"(b[1]),
-		"d"(b[2]), "d"(b[3]));
+	asm volatile("mma.sync.aligned.m16n8k4.row.col.f64.f64.f64.f64 {%0, %1, %2, %3}, {%4, %5}, {%6}, {%0, %1, %2, %3};"
+		: "+d"(c[0]), "+d"(c[1]), "+d"(c[2]), "+d"(c[3]) : "d"(a0), "d"(a1), "d"(b));
 }
 
 template <int I>
@@ -69,32 +69,32 @@ __device__ __forceinline__ void AssembleRow(AssembleShared& sm, const double* __
 			for (int t = 0; t < kFeatures; ++t) ph[t] = __ldg(p+(size_t)t*kQuad*kMaxBasis);
 		}
 	};
-	auto stage = [&](int c, int buffer) {
+	auto stage = [&](int c, int slot) {
 		// Psi rows k = 4 point + s, sixteen rows of up to 32 16-byte units, two rows per warp; the numbers
 		#pragma unroll
 		for (int r = 0; r < 2; ++r) {
 			const int k = 2*warp+r;
 			if (2*lane < columns) {
-				const uint32_t dst = (uint32_t)__cvta_generic_to_shared(&sm.Psi[buffer][k][2*lane]);
+				const uint32_t dst = (uint32_t)__cvta_generic_to_shared(&sm.Psi[slot][k][2*lane]);
 				const double* src = P+((size_t)(k & 3)*kQuad+c*kChunkPoints+(k >> 2))*kMaxBasis+2*lane;
 				asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" :: "r"(dst), "l"(src) : "memory");
 			}
 		}
 		if (tid < kChunkPoints*kPack/2) {
-			const uint32_t dst = (uint32_t)__cvta_generic_to_shared(&sm.pack[buffer][0][0]+2*tid);
+			const uint32_t dst = (uint32_t)__cvta_generic_to_shared(&sm.pack[slot][0][0]+2*tid);
 			asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" :: "r"(dst),
 				"l"(packs+(size_t)c*kChunkPoints*kPack+2*tid) : "memory");
 		}
 		asm volatile("cp.async.commit_group;" ::: "memory");
 	};
-	auto build = [&](int buffer) {
+	auto build = [&](int buffer, int slot) {
 		if (!builds) return;
-		const double* pk = sm.pack[buffer][point];
+		const double* pk = sm.pack[slot][point];
 		const auto coef = [&](int k) { return pk[k]; };
 		const double n = ph[0], g[3] = {ph[1], ph[2], ph[3]};
 		const double l = pk[kPackU]*g[0]+pk[kPackU+1]*g[1]+pk[kPackU+2]*g[2]-nu*ph[4];
 		auto put = [&](int f, const double v[4]) {
-			double2* d = reinterpret_cast<double2*>(&sm.G[buffer][4*lane+f][4*point]);
+			double2* d = reinterpret_cast<double2*>(&sm.G[buffer][lane*kGFunction+f*kGStride+4*point]);
 			d[0] = make_double2(v[0], v[1]);
 			d[1] = make_double2(v[2], v[3]);
 		};
@@ -111,65 +111,79 @@ __device__ __forceinline__ void AssembleRow(AssembleShared& sm, const double* __
 			put(3, v);
 		}
 	};
-	constexpr int kTiles = kMaxBasis/8;
+	// The product's 16 x 8 tiles, row tile by row tile, in even runs over the eight warps: whole row tiles per
+	// warp would leave two of the four schedulers half idle at 48 functions (six row tiles).
+	constexpr int kTiles = kMaxBasis/8;          // tiles per warp at most
+	const int across = columns >> 3, tiles = ((bn+3) >> 2)*across;
+	const int tile0 = warp*tiles/8, mine = (warp+1)*tiles/8-tile0;
+	const int m0 = tile0/across, n0 = tile0-m0*across;
 	double acc[kTiles][4];
 	#pragma unroll
 	for (int t = 0; t < kTiles; ++t)
 		#pragma unroll
 		for (int k = 0; k < 4; ++k) acc[t][k] = 0.0;
 	const int gr = lane >> 2, t4 = lane & 3;
-	const bool multiplies = 4*warp < bn;         // this warp's sixteen rows: functions 4 warp .. 4 warp + 3
 	constexpr int kChunks = kQuad/kChunkPoints;
 	load(0);
 	stage(0, 0);
-	asm volatile("cp.async.wait_group 0;" ::: "memory");
-	__syncthreads();
-	build(0);
-	load(1);
 	stage(1, 1);
-	for (int c = 0; c < kChunks; ++c) {
-		const int buffer = c & 1;
+	asm volatile("cp.async.wait_group 1;" ::: "memory");
+	__syncthreads();
+	build(0, 0);
+	load(1);
+	for (int c = 0, slot = 0; c < kChunks; ++c) {
+		const double* g_row = sm.G[c & 1]+(gr >> 2)*kGFunction+(gr & 3)*kGStride;
+		const int buffer = c & 1, next = slot == 2 ? 0 : slot+1, after = next == 2 ? 0 : next+1;
 		asm volatile("cp.async.wait_group 0;" ::: "memory");
-		__syncthreads();                         // G and Psi of chunk c, numbers and Psi of chunk c + 1
-		if (c+1 < kChunks) build(buffer^1);
+		__syncthreads();                         // G of chunk c; numbers and Psi of chunk c + 1; chunk c - 1's are free
+		if (c+2 < kChunks) stage(c+2, after);
+		if (c+1 < kChunks) build(buffer^1, next);
 		if (c+2 < kChunks) load(c+2);
-		if (multiplies) {
-			double a[8];
-			#pragma unroll
-			for (int j = 0; j < 4; ++j) {
-				a[2*j] = sm.G[buffer][16*warp+gr][4*j+t4];
-				a[2*j+1] = sm.G[buffer][16*warp+gr+8][4*j+t4];
-			}
-			#pragma unroll
-			for (int t = 0; t < kTiles; ++t)
-				if (8*t < columns) {
-					double b[4];
-					#pragma unroll
-					for (int j = 0; j < 4; ++j) b[j] = sm.Psi[buffer][4*j+t4][8*t+gr];
-					Mma16816(acc[t], a, b);
-				}
-		}
-		__syncthreads();                         // chunk c's buffers are free
-		if (c+2 < kChunks) stage(c+2, buffer);
-	}
-	// rows gr and gr + 8 are (function 4 warp + gr / 4 [+ 2], field gr % 4), columns 8 t + 2 t4 [+ 1] functions a:
-	// four lanes add one block row of a block, 32 contiguous bytes
-	if (!multiplies) return;
-	#pragma unroll
-	for (int h = 0; h < 2; ++h) {
-		const int bl = 4*warp+(gr >> 2)+2*h;
-		if (bl >= bn) continue;
-		const int b = b0+bl;
+		double a[8];
+		int m = m0, n = n0;
 		#pragma unroll
-		for (int t = 0; t < kTiles; ++t) {
-			#pragma unroll
-			for (int k = 0; k < 2; ++k) {
-				const int a = 8*t+2*t4+k;
-				const int block = a < nen ? EB[a*kMaxBasis+b] : -1;
-				if (block >= 0) atomicAdd(values+(size_t)block*16+I*4+(gr & 3), acc[t][2*h+k]);
+		for (int t = 0; t < kTiles; ++t)
+			if (t < mine) {
+				if (t == 0 || n == 0) {
+					#pragma unroll
+					for (int j = 0; j < 4; ++j) {
+						a[2*j] = g_row[(4*m)*kGFunction+4*j+t4];
+						a[2*j+1] = g_row[(4*m+2)*kGFunction+4*j+t4];
+					}
+				}
+				double b[4];
+				#pragma unroll
+				for (int j = 0; j < 4; ++j) b[j] = sm.Psi[slot][4*j+t4][8*n+gr];
+				#pragma unroll
+				for (int j = 0; j < 4; ++j) Mma1684(acc[t], a[2*j], a[2*j+1], b[j]);
+				if (++n == across) { n = 0; ++m; }
 			}
-		}
+		slot = next;
 	}
+	// rows gr and gr + 8 of row tile m are (function 4 m + gr / 4 [+ 2], field gr % 4), columns 8 n + 2 t4 [+ 1]
+	// functions a: four lanes add one block row of a block, 32 contiguous bytes
+	// (block indices fetched a tile ahead of the additions)
+	auto blocks_of = [&](int m, int n, int out[4]) {
+		#pragma unroll
+		for (int u = 0; u < 4; ++u) {
+			const int bl = 4*m+(gr >> 2)+2*(u >> 1), a = 8*n+2*t4+(u & 1);
+			out[u] = a < nen && bl < bn ? __ldg(EB+a*kMaxBasis+b0+bl) : -1;
+		}
+	};
+	int m = m0, n = n0, block[4];
+	if (mine > 0) blocks_of(m, n, block);
+	#pragma unroll
+	for (int t = 0; t < kTiles; ++t)
+		if (t < mine) {
+			if (++n == across) { n = 0; ++m; }
+			int ahead[4];
+			if (t+1 < mine) blocks_of(m, n, ahead);
+			#pragma unroll
+			for (int u = 0; u < 4; ++u)
+				if (block[u] >= 0) atomicAdd(values+(size_t)block[u]*16+I*4+(gr & 3), acc[t][u]);
+			#pragma unroll
+			for (int u = 0; u < 4; ++u) block[u] = ahead[u];
+		}
 }
 
 __global__ void __launch_bounds__(kThreads, 2) AssembleKernel(DeviceMeshView mesh, int first,
@@ -181,7 +195,7 @@ __global__ void __launch_bounds__(kThreads, 2) AssembleKernel(DeviceMeshView mes
 	const int local = blockIdx.x >> 3, row = (blockIdx.x >> 1) & 3, half = blockIdx.x & 1;
 	const int e = first+local;
 	const int nen = mesh.element_offsets[e+1]-mesh.element_offsets[e];
-	// the functions b in two even parts of whole warps' rows, one part where 32 hold them all
+	// the functions b in two even parts of whole row tiles, one part where 32 hold them all
 	const int part = nen > kHalf ? (nen+7)/8*4 : nen;
 	const int b0 = half*part, bn = min(part, nen-b0);
 	if (bn <= 0) return;

@@ -3,15 +3,17 @@
 // Formulation: vms_point.cuh (residual) and vms_tangent.cuh (the tangent's numbers), FP64 throughout.
 //
 // What bounds it: the tables, 164 KB per element, read once.  A CTA of 128 threads owns an element and
-// streams its points in eight chunks of eight; the chunk after next is fetched (cp.async, the columns of
-// the element's own functions only) while one is worked on.  Per chunk: the state of the eight points is a
-// matrix product (8 points x functions x 8 fields per table) on the FP64 tensor path, the functions split
-// over the four warps; one warp then forms the stabilisation, the residual's and the tangent's numbers, a
-// lane per (point, row field); all threads add the chunk's share of the residual, a thread per function and
-// half of the points.  Points need every function and the residual every point, so a chunk of points is
-// the unit that reads each table entry once: the kernel it replaces read the tables twice and reduced 22
-// sums per point through shared memory.  Four CTAs per SM (54 KB of shared memory each) cover each
-// other's latencies.  12,800-element section (nen 27 .. 64): 1225 us before.
+// streams its points in eight chunks of eight (cp.async, the columns of the element's own functions only).
+// Points need every function and the residual every point, so a chunk of points is the unit that reads each
+// table entry once; the kernel it replaces read the tables twice and reduced 22 sums per point through
+// shared memory.  Per chunk:
+//   warp 0 forms the stabilisation, the residual's and the tangent's numbers, a lane per (point, row field),
+//   a chain of some hundred dependent FP64 operations, while
+//   warps 1 - 3 form the next chunk's state as a matrix product (8 points x functions x 8 fields per table)
+//   on the FP64 tensor path, the functions split over the warps;
+//   then all threads add the chunk's share of the residual, a thread per function and half of the points.
+// Four CTAs per SM (54 KB of shared memory each) cover each other's latencies.
+// 12,800-element section (nen 27 .. 64): 1225 us before; with the phases one after the other 660 us, now 547 us.
 #include "common.hpp"
 #include "kernels.cuh"
 #include "vms_tangent.cuh"
@@ -27,16 +29,20 @@ constexpr int kChunk = 8;                        // points per chunk
 constexpr int kChunks = kQuad/kChunk;
 constexpr int kRows = kFeatures*kChunk;          // table rows per chunk
 constexpr int kSums = 64+4*32;                   // state sums of a chunk: 8 points x (8 fields of N, 4 of the rest)
+constexpr int kStage = kPack+1;                  // row stride of a chunk's tangent numbers
+constexpr int kSumWarps = kWarps-1;              // warps that form the next chunk's state
 
 struct Shared {
 	double ring[2][kRows][kMaxBasis];
-	double U[kMaxBasis*8];                       // state (4) and previous velocity (3) of every function
-	double part[kWarps][kSums];
+	// state (4) and previous velocity (3) of every function, until the warps hold theirs; then the chunk's
+	// tangent numbers, and at the end the residual of the second half of the points
+	double stage[kChunk*kStage];
+	double part[kSumWarps][kSums];
 	double sums[kSums];
 	double rc[kChunk][4][4];                     // [point][test feature][row field]
+	double qd[2][kChunk*kQData];
 };
-constexpr int kStage = kPack+1;                  // the tangent's numbers of a chunk, in place of `part`
-static_assert(kChunk*kStage <= kWarps*kSums, "the staged numbers fit the partial sums' place");
+static_assert(kMaxBasis*8 <= kChunk*kStage, "the functions' states fit the staged numbers' place");
 
 // Entry a of a staged row: 16-byte units are swizzled by the point so that eight rows' equal columns lie in
 // different banks.
@@ -51,13 +57,18 @@ __device__ __forceinline__ void Mma884(double& c0, double& c1, double a, double 
 		: "+d"(c0), "+d"(c1) : "d"(a), "d"(b));
 }
 
+// Material and time step with the quotients that every point uses (idt 0: steady).
+struct PointParams {
+	double rho, mu, nu, irho, idt;
+};
+
 // One (point, row field): residual numbers rc[test feature] and the row's tangent numbers into `pack`.
 template <bool kTangent>
-__device__ __forceinline__ void PointRow(int i, const double* sums, int q, const double* qd, const AssemblyParams& prm,
+__device__ __forceinline__ void PointRow(int i, const double* sums, int q, const double* qd, const PointParams& prm,
 	double rc[4], double* pack)
 {
-	const double rho = prm.density, mu = prm.viscosity, nu = mu/rho, dt = prm.dt;
-	const double idt = dt > 0.0 ? 1.0/dt : 0.0, irho = 1.0/rho;
+	const double rho = prm.rho, mu = prm.mu, nu = prm.nu, idt = prm.idt, irho = prm.irho;
+	const double inverse_direction = 1.0/qd[7];
 	double u[3], up[3], gv[3][3], gp[3], lap[3];
 	#pragma unroll
 	for (int c = 0; c < 3; ++c) {
@@ -76,11 +87,12 @@ __device__ __forceinline__ void PointRow(int i, const double* sums, int q, const
 	for (int f = 0; f < 3; ++f) {
 		Gu[f] = G[f][0]*u[0]+G[f][1]*u[1]+G[f][2]*u[2];
 		vm += u[f]*Gu[f];
-		dudt[f] = dt > 0.0 ? (u[f]-up[f])*idt : 0.0;
+		dudt[f] = (u[f]-up[f])*idt;
 	}
-	const double temporal = dt > 0.0 ? 4.0*idt*idt : 0.0;
-	const double tau_m = 1.0/sqrt(temporal+vm+(1.0/12.0)*nu*nu*qd[8]);
-	const double tau_c = 1.0/(tau_m*qd[7]);
+	// tau_M = S^(-1/2), tau_C = 1 / (tau_M |direction|^2) = S tau_M / |direction|^2
+	const double S = 4.0*idt*idt+vm+(1.0/12.0)*nu*nu*qd[8];
+	const double tau_m = rsqrt(S);
+	const double tau_c = S*tau_m*inverse_direction;
 	double R[3], fine[3], a[3];
 	#pragma unroll
 	for (int c = 0; c < 3; ++c) {
@@ -154,11 +166,11 @@ __device__ __forceinline__ void PointRow(int i, const double* sums, int q, const
 template <class C>
 __global__ void __launch_bounds__(kThreads, 4) PointStreamKernel(DeviceMeshView mesh, int first,
 	const double* __restrict__ phi, const double* __restrict__ qdata, const double* __restrict__ state,
-	const double* __restrict__ previous, AssemblyParams prm, C* __restrict__ packs, double* __restrict__ rhs)
+	const double* __restrict__ previous, PointParams prm, C* __restrict__ packs, double* __restrict__ rhs)
 {
 	extern __shared__ __align__(16) unsigned char raw[];
 	Shared& sm = *reinterpret_cast<Shared*>(raw);
-	double* stage = &sm.part[0][0];
+	double* U = sm.stage;
 	constexpr bool kTangent = !std::is_same<C, void>::value;
 	const int e = first+blockIdx.x;
 	const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -167,15 +179,24 @@ __global__ void __launch_bounds__(kThreads, 4) PointStreamKernel(DeviceMeshView 
 	const int columns = (nen+3) & ~3;                // the tables are zero past nen
 	const double* P = phi+(size_t)e*kFeatures*kQuad*kMaxBasis;
 
+	// Warps 1 - 3 fetch: they need the next chunk's rows while warp 0 is still with the last one's numbers.
 	auto fetch = [&](int c, int buffer) {
+		if (warp == 0) return;
 		if (2*lane < columns) {
 			#pragma unroll
-			for (int r0 = 0; r0 < kRows; r0 += kWarps) {
-				const int r = r0+warp, t = r/kChunk, q = r%kChunk;
-				const uint32_t dst = (uint32_t)__cvta_generic_to_shared(&sm.ring[buffer][r][Column(q, 2*lane)]);
-				const double* src = P+((size_t)t*kQuad+c*kChunk+q)*kMaxBasis+2*lane;
-				asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" :: "r"(dst), "l"(src) : "memory");
+			for (int r0 = 0; r0 < kRows; r0 += kSumWarps) {
+				const int r = r0+warp-1, t = r/kChunk, q = r%kChunk;
+				if (r < kRows) {
+					const uint32_t dst = (uint32_t)__cvta_generic_to_shared(&sm.ring[buffer][r][Column(q, 2*lane)]);
+					const double* src = P+((size_t)t*kQuad+c*kChunk+q)*kMaxBasis+2*lane;
+					asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" :: "r"(dst), "l"(src) : "memory");
+				}
 			}
+		}
+		if (tid-32 < kChunk*kQData/2) {
+			const uint32_t dst = (uint32_t)__cvta_generic_to_shared(&sm.qd[buffer][2*(tid-32)]);
+			const double* src = qdata+((size_t)e*kQuad+c*kChunk)*kQData+2*(tid-32);
+			asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" :: "r"(dst), "l"(src) : "memory");
 		}
 		asm volatile("cp.async.commit_group;" ::: "memory");
 	};
@@ -189,56 +210,69 @@ __global__ void __launch_bounds__(kThreads, 4) PointStreamKernel(DeviceMeshView 
 			const double2 x01 = *reinterpret_cast<const double2*>(state+4*node);
 			const double2 x23 = *reinterpret_cast<const double2*>(state+4*node+2);
 			v[0] = x01.x; v[1] = x01.y; v[2] = x23.x; v[3] = x23.y;
-			if (prm.dt > 0.0) {
+			if (prm.idt > 0.0) {
 				const double2 y01 = *reinterpret_cast<const double2*>(previous+4*node);
 				v[4] = y01.x; v[5] = y01.y; v[6] = previous[4*node+2];
 			}
 		}
 		#pragma unroll
-		for (int f = 0; f < 8; ++f) sm.U[tid*8+f] = v[f];
+		for (int f = 0; f < 8; ++f) U[tid*8+f] = v[f];
 	}
 	__syncthreads();
-	// this warp's functions: steps of four, warp, warp + 4, ...
+	// the functions of warps 1 - 3: steps of four, warp - 1, warp + 2, ...
+	constexpr int kSteps = (kMaxBasis/4+kSumWarps-1)/kSumWarps;
 	const int g = lane >> 2, t4 = lane & 3;
 	const int steps = columns >> 2;
-	double ub[4];
+	double ub[kSteps];
 	#pragma unroll
-	for (int m = 0; m < 4; ++m) ub[m] = sm.U[(4*(warp+4*m)+t4)*8+g];
+	for (int m = 0; m < kSteps; ++m) {
+		const int s = warp-1+kSumWarps*m;
+		ub[m] = warp > 0 && s < steps ? U[(4*s+t4)*8+g] : 0.0;
+	}
 	double res[4] = {0.0, 0.0, 0.0, 0.0};
 	const int a = tid & 63, half = tid >> 6;
 
-	for (int c = 0; c < kChunks; ++c) {
-		const int buffer = c & 1;
-		if (c+1 < kChunks) asm volatile("cp.async.wait_group 1;" ::: "memory");
-		else asm volatile("cp.async.wait_group 0;" ::: "memory");
-		__syncthreads();
+	auto form_state = [&](int buffer) {
 		double acc[kFeatures][2];
 		#pragma unroll
 		for (int t = 0; t < kFeatures; ++t) acc[t][0] = acc[t][1] = 0.0;
 		#pragma unroll
-		for (int m = 0; m < 4; ++m) {
-			const int s = warp+4*m;
+		for (int m = 0; m < kSteps; ++m) {
+			const int s = warp-1+kSumWarps*m;
 			if (s < steps) {
 				#pragma unroll
 				for (int t = 0; t < kFeatures; ++t)
 					Mma884(acc[t][0], acc[t][1], sm.ring[buffer][t*kChunk+g][Column(g, 4*s+t4)], ub[m]);
 			}
 		}
-		*reinterpret_cast<double2*>(&sm.part[warp][8*g+2*t4]) = make_double2(acc[0][0], acc[0][1]);
+		double* part = sm.part[warp-1];
+		*reinterpret_cast<double2*>(&part[8*g+2*t4]) = make_double2(acc[0][0], acc[0][1]);
 		if (t4 < 2) {
 			#pragma unroll
 			for (int t = 1; t < kFeatures; ++t)
-				*reinterpret_cast<double2*>(&sm.part[warp][64+32*(t-1)+4*g+2*t4]) = make_double2(acc[t][0], acc[t][1]);
+				*reinterpret_cast<double2*>(&part[64+32*(t-1)+4*g+2*t4]) = make_double2(acc[t][0], acc[t][1]);
 		}
-		__syncthreads();
-		for (int k = tid; k < kSums; k += kThreads)
-			sm.sums[k] = (sm.part[0][k]+sm.part[1][k])+(sm.part[2][k]+sm.part[3][k]);
-		__syncthreads();
+	};
+	auto add_parts = [&]() {
+		for (int k = tid; k < kSums; k += kThreads) sm.sums[k] = (sm.part[0][k]+sm.part[1][k])+sm.part[2][k];
+	};
+	asm volatile("cp.async.wait_group 1;" ::: "memory");
+	__syncthreads();
+	if (warp > 0) form_state(0);
+	__syncthreads();
+	add_parts();
+	__syncthreads();
+	for (int c = 0; c < kChunks; ++c) {
+		const int buffer = c & 1;
 		if (warp == 0) {
 			double rc[4];
-			PointRow<kTangent>(t4, sm.sums, g, qdata+((size_t)e*kQuad+c*kChunk+g)*kQData, prm, rc, stage+g*kStage);
+			PointRow<kTangent>(t4, sm.sums, g, &sm.qd[buffer][g*kQData], prm, rc, sm.stage+g*kStage);
 			#pragma unroll
 			for (int s = 0; s < 4; ++s) sm.rc[g][s][t4] = rc[s];
+		} else if (c+1 < kChunks) {
+			asm volatile("cp.async.wait_group 0;" ::: "memory");
+			asm volatile("bar.sync 1, %0;" :: "n"(32*kSumWarps) : "memory");   // chunk c + 1's rows
+			form_state(buffer^1);
 		}
 		__syncthreads();
 		if (rhs != nullptr && a < nen) {
@@ -255,29 +289,33 @@ __global__ void __launch_bounds__(kThreads, 4) PointStreamKernel(DeviceMeshView 
 				}
 			}
 		}
+		// a warp per two points
 		if constexpr (std::is_same<C, double>::value) {
-			double* out = packs+((size_t)blockIdx.x*kQuad+c*kChunk)*kPack;
-			for (int k = tid; k < kChunk*kPack; k += kThreads) out[k] = stage[(k/kPack)*kStage+k%kPack];
-		} else if constexpr (std::is_same<C, float>::value) {
-			float2* out = reinterpret_cast<float2*>(packs+((size_t)blockIdx.x*kQuad+c*kChunk)*kPack);
-			for (int k = tid; k < kChunk/2*kPack; k += kThreads) {
-				const int pair = k/kPack, n = k%kPack;
-				out[k] = make_float2((float)stage[2*pair*kStage+n], (float)stage[(2*pair+1)*kStage+n]);
+			double* out = packs+((size_t)blockIdx.x*kQuad+c*kChunk+2*warp)*kPack;
+			const double* in = sm.stage+2*warp*kStage;
+			for (int k = lane; k < kPack; k += 32) {
+				out[k] = in[k];
+				out[kPack+k] = in[kStage+k];
 			}
+		} else if constexpr (std::is_same<C, float>::value) {
+			float2* out = reinterpret_cast<float2*>(packs+((size_t)blockIdx.x*kQuad+c*kChunk+2*warp)*kPack);
+			const double* in = sm.stage+2*warp*kStage;
+			for (int k = lane; k < kPack; k += 32) out[k] = make_float2((float)in[k], (float)in[kStage+k]);
 		}
-		__syncthreads();
+		if (c+1 < kChunks) add_parts();
+		__syncthreads();                             // chunk c's rows and numbers are free, chunk c + 1's sums there
 		if (c+2 < kChunks) fetch(c+2, buffer);
 	}
 	if (rhs == nullptr) return;
 	// the two halves of the points, then into the nodes
 	if (half == 1)
 		#pragma unroll
-		for (int f = 0; f < 4; ++f) sm.part[0][4*a+f] = res[f];
+		for (int f = 0; f < 4; ++f) sm.stage[4*a+f] = res[f];
 	__syncthreads();
 	if (half == 0 && a < nen) {
 		double* r = rhs+4*(size_t)mesh.connectivity[begin+a];
 		#pragma unroll
-		for (int f = 0; f < 4; ++f) atomicAdd(r+f, res[f]+(&sm.part[0][0])[4*a+f]);
+		for (int f = 0; f < 4; ++f) atomicAdd(r+f, res[f]+sm.stage[4*a+f]);
 	}
 }
 
@@ -287,7 +325,9 @@ void Launch(const DeviceMeshView& mesh, int first, int count, const double* phi,
 {
 	CudaCheck(cudaFuncSetAttribute(PointStreamKernel<C>, cudaFuncAttributeMaxDynamicSharedMemorySize,
 		(int)sizeof(Shared)), "point kernel shared memory");
-	PointStreamKernel<C><<<count, kThreads, sizeof(Shared), stream>>>(mesh, first, phi, qdata, state, previous, params,
+	const PointParams prm{params.density, params.viscosity, params.viscosity/params.density, 1.0/params.density,
+		params.dt > 0.0 ? 1.0/params.dt : 0.0};
+	PointStreamKernel<C><<<count, kThreads, sizeof(Shared), stream>>>(mesh, first, phi, qdata, state, previous, prm,
 		packs, rhs);
 	LaunchCheck("PointStreamKernel");
 }
