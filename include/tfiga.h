@@ -136,18 +136,14 @@ typedef struct tfiga_ns_params {
 	 * before the tangent, so a converged check assembles no tangent), so only the
 	 * Newton convergence rate can change.  Default 0 (off). */
 	double tangent_reuse_factor;   /* default 0 */
-	/* Tensor-core modes: how the tangent's operands reach the tensor cores.
-	 * TFIGA_TANGENT_COEFFICIENTS: the point kernel stores every element's point
-	 * coefficients (80 KiB per element) and an FP32 copy of the basis tables is kept;
-	 * TFIGA_TANGENT_FUSED: the point kernel stores the FP64 point state (11 KiB per
-	 * element) and the tensor-core kernel makes the coefficients itself and stages
-	 * the basis from the FP64 tables (about 96 KiB per element less);
-	 * TFIGA_TANGENT_ELEMENT: the arrays of TFIGA_TANGENT_COEFFICIENTS contracted by one
-	 * persistent CTA per SM that takes whole elements (all four row fields at once, the
-	 * basis staged once per element);
-	 * TFIGA_TANGENT_AUTO: the first tangent assembly times the three (the two
-	 * coefficient-array ones when their memory is free) and keeps the fastest; the
-	 * fused one otherwise.
+	/* Tensor-core modes: how the tangent's basis values reach the tensor cores, and how the work is
+	 * spread.  The point kernel stores 72 numbers per quadrature point (18 KiB per element) in all of them.
+	 * TFIGA_TANGENT_COEFFICIENTS: an FP32 copy of the basis tables (80 KiB per element) is kept; a CTA per
+	 * element and row field;
+	 * TFIGA_TANGENT_ELEMENT: the same copy, two persistent CTAs per SM that take element after element;
+	 * TFIGA_TANGENT_FUSED: no copy, the FP64 tables are converted on the way;
+	 * TFIGA_TANGENT_AUTO: the first tangent assembly times the three (those with the copy when its memory
+	 * is free) and keeps the fastest; the fused one otherwise.
 	 * All give the same tangent up to the order of the FP32 additions. */
 	int32_t tangent_kernel;        /* default TFIGA_TANGENT_AUTO */
 } tfiga_ns_params;
@@ -334,11 +330,10 @@ int tfiga_ns_set_segments(tfiga_ns* ns, const int64_t* node_offsets, int32_t cou
  * residual norm (either output may be NULL). */
 int tfiga_ns_segment_status(tfiga_ns* ns, int32_t* done, double* residuals);
 /* Tensor-core modes: the tangent organisation in use (*kernel: TFIGA_TANGENT_*, AUTO before the
- * first tangent) and the autotuner's times of the coefficient-array (row-field-pair kernel) and fused
- * organisations (ms, 0 when not timed).  No counterpart in the reference.  Any output may be NULL. */
+ * first tangent) and the autotuner's times of the coefficients and fused organisations (ms, 0 when
+ * not timed).  No counterpart in the reference.  Any output may be NULL. */
 int tfiga_ns_tangent_kernel(tfiga_ns* ns, int32_t* kernel, double* coefficients_ms, double* fused_ms);
-/* The autotuner's time of the element kernel (TFIGA_TANGENT_ELEMENT) on the coefficient arrays (ms, 0
- * when not timed). */
+/* The autotuner's time of the element organisation (TFIGA_TANGENT_ELEMENT) (ms, 0 when not timed). */
 int tfiga_ns_tangent_element_ms(tfiga_ns* ns, double* element_ms);
 /* Outward flow through each labelled boundary (IntegrateBoundaryFlow,
  * BoundaryFlow.hpp:165-200; MeasureFlowConvergence iga_cuda.cu:520-557). */

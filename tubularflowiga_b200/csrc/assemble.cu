@@ -51,6 +51,16 @@ __device__ __forceinline__ void Mma1684(double c[4], double a0, double a1, doubl
 		: "+d"(c[0]), "+d"(c[1]), "+d"(c[2]), "+d"(c[3]) : "d"(a0), "d"(a1), "d"(b));
 }
 
+struct PackReader {
+	const double* p;
+	__device__ __forceinline__ double operator()(int k) const { return p[k]; }
+	__device__ __forceinline__ Two<double> two(int k) const
+	{
+		const double2 v = *reinterpret_cast<const double2*>(p+k);
+		return {v.x, v.y};
+	}
+};
+
 template <int I>
 __device__ __forceinline__ void AssembleRow(AssembleShared& sm, const double* __restrict__ P,
 	const double* __restrict__ packs, const int32_t* __restrict__ EB, int nen, int b0, int bn, double irho, double nu,
@@ -90,7 +100,7 @@ __device__ __forceinline__ void AssembleRow(AssembleShared& sm, const double* __
 	auto build = [&](int buffer, int slot) {
 		if (!builds) return;
 		const double* pk = sm.pack[slot][point];
-		const auto coef = [&](int k) { return pk[k]; };
+		const PackReader coef{pk};
 		const double n = ph[0], g[3] = {ph[1], ph[2], ph[3]};
 		const double l = pk[kPackU]*g[0]+pk[kPackU+1]*g[1]+pk[kPackU+2]*g[2]-nu*ph[4];
 		auto put = [&](int f, const double v[4]) {

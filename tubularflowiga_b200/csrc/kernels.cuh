@@ -85,31 +85,15 @@ void LaunchAssembleLarge(const DeviceMeshView& mesh, int first, int count, const
 	double* rhs, cudaStream_t stream);
 
 // ---- tangent_tc.cu -----------------------------------------------------
-// Tensor-core tangent in two launches.  LaunchTangentPoint: FP64 point state,
-// the coefficients of all four row fields into coef (workspace of elements x 4
-// x 80 x 64 floats; null: residual only) and the FP64 residual ADDED into rhs
-// (= -r).
-// LaunchTangentTc: the tangent contracted on the tcgen05 tensor cores from
-// coef and phi32 (the FP32 copy of phi, Mesh::phi32), FP32 accumulation, ADDED
-// into the FP32 values; status bit 1 set if an MMA completion wait expired.
-// operands: TC_OPERANDS_BF16, TC_OPERANDS_SPLIT (hi + lo BF16) or TC_OPERANDS_TF32.
-// point_state (elements x 64 x 22 doubles, may be null): the point state for LaunchTangentTcFused
-// instead of the coefficients (coef and point_state are not both given).
-void LaunchTangentPoint(const DeviceMeshView& mesh, const double* phi, const double* qdata, const double* state,
-	const double* previous, AssemblyParams params, float* coef, double* point_state, double* rhs,
-	cudaStream_t stream);
+// The tangent contracted on the tcgen05 tensor cores from the points' numbers (LaunchPointStream's packs32 of all
+// elements) and the basis values (phi32, the FP32 copy of Mesh::phi32, or phi when that is null), FP32
+// accumulation, ADDED into the FP32 values; status bit 1 set if an MMA completion wait expired.
+// operands: TC_OPERANDS_BF16, TC_OPERANDS_SPLIT (hi + lo BF16) or TC_OPERANDS_TF32.  persistent: two CTAs per SM
+// take (element, row field) after (element, row field), instead of a CTA for each.
 enum : int { TC_OPERANDS_BF16 = 0, TC_OPERANDS_SPLIT = 1, TC_OPERANDS_TF32 = 2 };
-void LaunchTangentTc(const DeviceMeshView& mesh, const float* phi32, const float* coef,
-	const int32_t* element_blocks, float* values, int* status, int operands, cudaStream_t stream);
-// The same contraction with one persistent CTA per SM taking whole elements (all four row fields, the
-// basis chunk staged once per element; 512 TMEM columns, so one CTA per SM).
-void LaunchTangentTcElement(const DeviceMeshView& mesh, const float* phi32, const float* coef,
-	const int32_t* element_blocks, float* values, int* status, int operands, cudaStream_t stream);
-// The same contraction with the coefficients made in the kernel from the stored point state and the
-// basis staged from the FP64 tables (no coefficient array, no FP32 copy of the tables).
-void LaunchTangentTcFused(const DeviceMeshView& mesh, const double* phi, const double* qdata,
-	const double* point_state, AssemblyParams params, const int32_t* element_blocks, float* values, int* status,
-	int operands, cudaStream_t stream);
+void LaunchTangentTc(const DeviceMeshView& mesh, const float* phi32, const double* phi, const float* packs,
+	const int32_t* element_blocks, AssemblyParams params, float* values, int* status, int operands, bool persistent,
+	cudaStream_t stream);
 
 // ---- sparse.cu ----------------------------------------------------------
 // Matrix values are FP64 or FP32 (T = double / float); vectors are FP64.

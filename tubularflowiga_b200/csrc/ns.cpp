@@ -88,8 +88,7 @@ NsSolver::NsSolver(Mesh& mesh, const tfiga_ns_params& params)
 	tangent_kernel_ = params.tangent_kernel;
 	if (tensor_tangent()) {
 		const size_t regular = (size_t)mesh.regular_elements();
-		if (coefficient_arrays()) coef32_.Allocate(regular*4*80*64);
-		else point_state_.Allocate(regular*kQuad*22);
+		packs32_.Allocate(regular*kQuad*kPointNumbers);
 	}
 	if (tensor_tangent()) {
 		status_.Allocate(1);
@@ -212,10 +211,8 @@ void NsSolver::AssembleResidualTc()
 	rhs_.Zero(stream_);
 	profiler_.End(stream_);
 	profiler_.Begin(Profiler::kResidual, stream_);
-	const bool coefficients = coefficient_arrays();
-	LaunchTangentPoint(mesh_.regular_view(), mesh_.phi(), mesh_.qdata(), state_.get(), previous_.get(),
-		{params_.density, params_.viscosity, params_.dt}, coefficients ? coef32_.get() : nullptr,
-		coefficients ? nullptr : point_state_.get(), rhs_.get(), stream_);
+	LaunchPointStream(mesh_.regular_view(), 0, (int)mesh_.regular_elements(), mesh_.phi(), mesh_.qdata(), state_.get(),
+		previous_.get(), {params_.density, params_.viscosity, params_.dt}, nullptr, packs32_.get(), rhs_.get(), stream_);
 	LargeElements<float>(nullptr, rhs_.get());
 	profiler_.End(stream_);
 	profiler_.Begin(Profiler::kVector, stream_);
@@ -234,27 +231,21 @@ void NsSolver::LargeElements(T* values, double* rhs)
 	launches_ += 1;
 }
 
+void NsSolver::LaunchTangent(int organisation)
+{
+	values32_.Zero(stream_);
+	LaunchTangentTc(mesh_.regular_view(), organisation == TFIGA_TANGENT_FUSED ? nullptr : mesh_.phi32(), mesh_.phi(),
+		packs32_.get(), mesh_.element_blocks(), {params_.density, params_.viscosity, params_.dt}, values32_.get(),
+		status_.get(), tc_operands(), organisation == TFIGA_TANGENT_ELEMENT, stream_);
+	launches_ += 1;
+}
+
 void NsSolver::AssembleTangentTc()
 {
 	amg_current_ = false;
-	const int operands = tc_operands();
-	const AssemblyParams prm{params_.density, params_.viscosity, params_.dt};
 	profiler_.Begin(Profiler::kAssembly, stream_);
-	if (tangent_kernel_ == TFIGA_TANGENT_AUTO) {
-		AutotuneTangent();
-	} else {
-		values32_.Zero(stream_);
-		if (tangent_kernel_ == TFIGA_TANGENT_FUSED)
-			LaunchTangentTcFused(mesh_.regular_view(), mesh_.phi(), mesh_.qdata(), point_state_.get(), prm,
-				mesh_.element_blocks(), values32_.get(), status_.get(), operands, stream_);
-		else if (tangent_kernel_ == TFIGA_TANGENT_ELEMENT)
-			LaunchTangentTcElement(mesh_.regular_view(), mesh_.phi32(), coef32_.get(), mesh_.element_blocks(),
-				values32_.get(), status_.get(), operands, stream_);
-		else
-			LaunchTangentTc(mesh_.regular_view(), mesh_.phi32(), coef32_.get(), mesh_.element_blocks(),
-				values32_.get(), status_.get(), operands, stream_);
-		launches_ += 1;
-	}
+	if (tangent_kernel_ == TFIGA_TANGENT_AUTO) AutotuneTangent();
+	else LaunchTangent(tangent_kernel_);
 	LargeElements<float>(values32_.get(), nullptr);
 	profiler_.End(stream_);
 	if (amg_ && !amg_->built()) amg_->Build(values32_.get());
@@ -262,70 +253,37 @@ void NsSolver::AssembleTangentTc()
 
 void NsSolver::AutotuneTangent()
 {
-	const int operands = tc_operands();
-	const AssemblyParams prm{params_.density, params_.viscosity, params_.dt};
-	const DeviceMeshView view = mesh_.regular_view();
-	cudaEvent_t ev[4];
+	cudaEvent_t ev[2];
 	for (auto& e : ev) CudaCheck(cudaEventCreate(&e), "autotune event");
 	struct Events {
 		cudaEvent_t* e;
-		~Events() { for (int i = 0; i < 4; ++i) cudaEventDestroy(e[i]); }
+		~Events() { for (int i = 0; i < 2; ++i) cudaEventDestroy(e[i]); }
 	} guard{ev};
-	// the fused organisation first: the residual pass has just stored its point state
-	values32_.Zero(stream_);
-	CudaCheck(cudaEventRecord(ev[0], stream_), "event");
-	LaunchTangentTcFused(view, mesh_.phi(), mesh_.qdata(), point_state_.get(), prm, mesh_.element_blocks(),
-		values32_.get(), status_.get(), operands, stream_);
-	CudaCheck(cudaEventRecord(ev[1], stream_), "event");
-	launches_ += 1;
-	CudaCheck(cudaStreamSynchronize(stream_), "tangent autotune");
-	float ms = 0.0f;
-	CudaCheck(cudaEventElapsedTime(&ms, ev[0], ev[1]), "event time");
-	tune_ms_[1] = ms;
-	// the coefficient-array organisation, when its arrays fit with 2 GiB to spare
-	const size_t regular = (size_t)mesh_.regular_elements();
-	const size_t need = regular*4*80*64*sizeof(float)+regular*kFeatures*kQuad*kMaxBasis*sizeof(float);
+	auto timed = [&](int organisation) {
+		CudaCheck(cudaEventRecord(ev[0], stream_), "event");
+		LaunchTangent(organisation);
+		CudaCheck(cudaEventRecord(ev[1], stream_), "event");
+		CudaCheck(cudaStreamSynchronize(stream_), "tangent autotune");
+		float ms = 0.0f;
+		CudaCheck(cudaEventElapsedTime(&ms, ev[0], ev[1]), "event time");
+		return (double)ms;
+	};
+	tune_ms_[1] = timed(TFIGA_TANGENT_FUSED);
+	tangent_kernel_ = TFIGA_TANGENT_FUSED;
+	// the organisations with an FP32 copy of the basis tables, when it fits with 2 GiB to spare (or is there)
+	const size_t need = (size_t)mesh_.regular_elements()*kFeatures*kQuad*kMaxBasis*sizeof(float);
 	size_t free_bytes = 0, total_bytes = 0;
 	CudaCheck(cudaMemGetInfo(&free_bytes, &total_bytes), "device memory");
-	if (free_bytes < need+(size_t(2) << 30)) {
-		tangent_kernel_ = TFIGA_TANGENT_FUSED;
-		return;
-	}
-	coef32_.Allocate(regular*4*80*64);
-	// the same state's coefficients; the residual this pass adds goes to the Newton update vector,
-	// which the linear solve clears before use
-	LaunchTangentPoint(view, mesh_.phi(), mesh_.qdata(), state_.get(), previous_.get(), prm, coef32_.get(), nullptr,
-		update_.get(), stream_);
-	const float* phi32 = mesh_.phi32();
-	values32_.Zero(stream_);
-	CudaCheck(cudaEventRecord(ev[2], stream_), "event");
-	LaunchTangentTc(view, phi32, coef32_.get(), mesh_.element_blocks(), values32_.get(), status_.get(), operands,
-		stream_);
-	CudaCheck(cudaEventRecord(ev[3], stream_), "event");
-	launches_ += 2;
-	CudaCheck(cudaStreamSynchronize(stream_), "tangent autotune");
-	CudaCheck(cudaEventElapsedTime(&ms, ev[2], ev[3]), "event time");
-	tune_ms_[0] = ms;
-	// the same arrays contracted element by element (its tangent, equal to the others' up to the order
-	// of the FP32 additions, is the one kept)
-	values32_.Zero(stream_);
-	CudaCheck(cudaEventRecord(ev[2], stream_), "event");
-	LaunchTangentTcElement(view, phi32, coef32_.get(), mesh_.element_blocks(), values32_.get(), status_.get(),
-		operands, stream_);
-	CudaCheck(cudaEventRecord(ev[3], stream_), "event");
-	launches_ += 1;
-	CudaCheck(cudaStreamSynchronize(stream_), "tangent autotune");
-	CudaCheck(cudaEventElapsedTime(&ms, ev[2], ev[3]), "event time");
-	tune_ms_[2] = ms;
-	const double arrays_ms = std::min(tune_ms_[0], tune_ms_[2]);
-	if (arrays_ms < tune_ms_[1]) {
-		tangent_kernel_ = tune_ms_[2] <= tune_ms_[0] ? TFIGA_TANGENT_ELEMENT : TFIGA_TANGENT_COEFFICIENTS;
-		point_state_.Release();
-	} else {
-		tangent_kernel_ = TFIGA_TANGENT_FUSED;
-		coef32_.Release();
+	if (!mesh_.has_phi32() && free_bytes < need+(size_t(2) << 30)) return;
+	const bool had = mesh_.has_phi32();
+	mesh_.phi32();
+	// (the last one's tangent, equal to the others' up to the order of the FP32 additions, is kept)
+	tune_ms_[2] = timed(TFIGA_TANGENT_ELEMENT);
+	tune_ms_[0] = timed(TFIGA_TANGENT_COEFFICIENTS);
+	if (std::min(tune_ms_[0], tune_ms_[2]) < tune_ms_[1])
+		tangent_kernel_ = tune_ms_[2] < tune_ms_[0] ? TFIGA_TANGENT_ELEMENT : TFIGA_TANGENT_COEFFICIENTS;
+	else if (!had)
 		mesh_.ReleasePhi32();
-	}
 }
 
 void NsSolver::AssembleResidual()
@@ -350,8 +308,9 @@ void NsSolver::AssembleResidual()
 
 void NsSolver::AssembleFp64(double* rhs)
 {
-	// in slabs of elements, whose points' numbers (36 KiB per element) share one workspace
-	constexpr int kSlab = 16384;
+	// in slabs of elements, whose points' numbers (36 KiB per element, 74 MB in all) share one workspace that the L2
+	// holds between the two kernels
+	constexpr int kSlab = 2048;
 	const int count = (int)mesh_.regular_elements();
 	const AssemblyParams prm{params_.density, params_.viscosity, params_.dt};
 	if (packs_.size() == 0) packs_.Allocate((size_t)std::min(kSlab, count)*kQuad*kPointNumbers);

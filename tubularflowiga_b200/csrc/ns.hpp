@@ -110,17 +110,16 @@ private:
 		double continuity_l2, continuity_sum, net_flow, absolute_flow, imbalance;
 	};
 	void ApplyTractions(const std::map<int32_t, double>& traction);
-	// Tensor-core modes: the FP64 residual and point coefficients (rhs = -r + traction), then the
-	// tangent from those coefficients into the FP32 Jacobian (builds the AMG on first use).
+	// Tensor-core modes: the FP64 residual and the points' numbers (rhs = -r + traction), then the
+	// tangent from those numbers into the FP32 Jacobian (builds the AMG on first use).
 	void AssembleResidualTc();
 	void ApplyDirichletParts(bool matrix, bool rhs);
 	void AssembleTangentTc();
-	// TFIGA_TANGENT_AUTO: times both tangent organisations on the current state (the separate one only
-	// when its arrays fit in free memory), keeps the faster and releases the other's arrays; values32_
-	// then holds the tangent.
+	// TFIGA_TANGENT_AUTO: times the tangent organisations on the current state (those with the FP32 basis
+	// copy only when it fits in free memory) and keeps the fastest; values32_ then holds the tangent.
 	void AutotuneTangent();
 	// Every mode, for the residual-first Newton iteration: the FP64 residual alone (rhs = -r +
-	// traction; in the tensor-core modes with the point coefficients), then -- only for an
+	// traction; in the tensor-core modes with the points' numbers), then -- only for an
 	// iteration that solves with a new tangent -- the Jacobian alone (FP64 assembly, or the
 	// tensor-core contraction; builds the AMG on first use).
 	void AssembleResidual();
@@ -153,15 +152,11 @@ private:
 	int64_t n4_;
 	DeviceArray<double> values_, rhs_, state_, previous_, update_, traction_, velocity_bc_, pressure_bc_;
 	DeviceArray<float> values32_;
-	DeviceArray<float> coef32_;              // tensor-core tangent: point coefficients [e][4][80][64]
+	DeviceArray<float> packs32_;             // tensor-core tangent: the points' numbers of every element
 	DeviceArray<double> packs_;              // FP64 tangent: the points' numbers of a slab of elements
-	DeviceArray<double> point_state_;        // fused tensor-core tangent: FP64 point state [e][64][22]
 	int tangent_kernel_ = 0;                 // TFIGA_TANGENT_* in use
-	double tune_ms_[3] = {0.0, 0.0, 0.0};    // autotuner: coefficient-array (pair), fused, element times
-	bool coefficient_arrays() const
-	{
-		return tangent_kernel_ == TFIGA_TANGENT_COEFFICIENTS || tangent_kernel_ == TFIGA_TANGENT_ELEMENT;
-	}
+	double tune_ms_[3] = {0.0, 0.0, 0.0};    // autotuner: coefficients, fused, element times
+	void LaunchTangent(int organisation);    // into values32_, cleared first
 	DeviceArray<double> face_flow_, face_pressure_, label_flow_, partial_, scalars_;
 	DeviceArray<int32_t> vmask_, pmask_, constrained_, face_slot_, status_;
 	std::vector<int32_t> labels_;            // distinct face labels (slot order)

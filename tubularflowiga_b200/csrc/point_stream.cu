@@ -136,12 +136,14 @@ __device__ __forceinline__ void PointRow(int i, const double* sums, int q, const
 		#pragma unroll
 		for (int f = 0; f < 3; ++f) {
 			const double Aif = i == 0 ? A[0][f] : i == 1 ? A[1][f] : A[2][f];
-			pack[kPackNN+3*i+f] = mr*(gi[f]+(f == i ? idt : 0.0)+A[0][f]*gi[0]+A[1][f]*gi[1]+A[2][f]*gi[2]);
-			pack[kPackTg+3*i+f] = mr*tau_m*gi[f];
+			double* column = pack+kPackColumn+6*(3*i+f);
+			column[0] = mr*(gi[f]+(f == i ? idt : 0.0)+A[0][f]*gi[0]+A[1][f]*gi[1]+A[2][f]*gi[2]);
+			column[1] = -mr*tau_m*gi[f];
 			const double dtau_c = tau_c*tau_m*tau_m*Gu[f];
 			#pragma unroll
 			for (int d = 0; d < 3; ++d)
-				pack[kPackC+9*i+3*f+d] = mr*((d == i ? dtau_c*divu : 0.0)-a[d]*Aif-fi*((d == f ? 1.0 : 0.0)+A[d][f]));
+				column[2+d] = mr*((d == i ? dtau_c*divu : 0.0)-a[d]*Aif-fi*((d == f ? 1.0 : 0.0)+A[d][f]));
+			column[5] = -meas*Aif;
 		}
 		pack[kPackPa+i] = mr*tau_m*ai;
 		pack[kPackPf+i] = mr*tau_m*fi;
@@ -153,11 +155,7 @@ __device__ __forceinline__ void PointRow(int i, const double* sums, int q, const
 		pack[kPackOne] = meas;
 		pack[kPackTau] = meas*tau_m;
 		pack[kPackTauRho] = meas*tau_m*irho;
-		#pragma unroll
-		for (int d = 0; d < 3; ++d)
-			#pragma unroll
-			for (int f = 0; f < 3; ++f) pack[kPackA+3*d+f] = meas*A[d][f];
-		pack[kPack-1] = 0.0;
+		pack[kPackMinusOne] = -meas;
 	}
 }
 

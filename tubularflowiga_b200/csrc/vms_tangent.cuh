@@ -6,7 +6,7 @@
 // (b, point).  Collecting the terms by their common factors
 //   L = u . grad N_b - nu Lap N_b   (the convection-diffusion operator of the strong residual),
 //   A = a . grad N_b                (a = u + fine-scale velocity)
-// leaves 71 numbers per point and about 130 products per (b, point) for all sixteen field pairs:
+// leaves 72 numbers per point and about 130 products per (b, point) for all sixteen field pairs:
 //   momentum row i, velocity column f:
 //     G_0     = nn_if N - tg_if L + [i = f] rho A
 //     G_{1+d} = c_ifd N + [i = f] (mu dN_d + pa_d L) + [d = i] rho tau_C dN_f + [d = f] (mu dN_i + pf_i L)
@@ -14,63 +14,84 @@
 //     G_0 = -(1/rho) tg_i . grad N,   G_{1+d} = -[d = i] N + (1/rho) (pa_d dN_i + pf_i dN_d)
 //   continuity row, velocity column f:  G_0 = dN_f,   G_{1+d} = -A_df N + [d = f] tau_M L
 //   continuity row, pressure column:    G_0 = 0,      G_{1+d} = (tau_M / rho) dN_d
-// All numbers carry the point's measure.
+// All numbers carry the point's measure; those that are subtracted are stored negated, so that a column is
+// multiplications and multiply-adds only.
 #pragma once
 
 #include "kernels.cuh"
 
 namespace tfiga {
 
-constexpr int kPack = kPointNumbers;             // numbers per point (one unused)
+constexpr int kPack = kPointNumbers;             // numbers per point
+// Ordered so that a column reads neighbours in pairs (every group starts at an even index).
 enum : int {
-	kPackNN = 0,        // [3 i + f]
-	kPackTg = 9,        // [3 i + f]  rho tau du_i/dx_f
-	kPackC = 18,        // [9 i + 3 f + d]
-	kPackPa = 45,       // [d]  rho tau a_d
-	kPackPf = 48,       // [i]  rho tau fine_i
-	kPackU = 51,        // [e]  u_e (without the measure)
-	kPackRa = 54,       // [e]  rho a_e
-	kPackMu = 57, kPackTauC = 58 /* rho tau_C */, kPackOne = 59 /* measure */, kPackTau = 60, kPackTauRho = 61,
-	kPackA = 62         // [3 d + f]
+	kPackColumn = 0,    // [6 (3 i + f)]: nn_if, -tg_if, c_if0, c_if1, c_if2, -A_if
+	kPackU = 54,        // [e]  u_e (without the measure)
+	kPackTau = 57,
+	kPackRa = 58,       // [e]  rho a_e
+	kPackMu = 61,
+	kPackPa = 62,       // [d]  rho tau a_d
+	kPackTauC = 65,     // rho tau_C
+	kPackPf = 66,       // [i]  rho tau fine_i
+	kPackOne = 69,      // measure
+	kPackMinusOne = 70,
+	kPackTauRho = 71
 };
 
-// G_0 .. G_3 of row field I and column field F.  coef(k): number k of the point; g: gradient of N_b, l: L.
+__device__ __forceinline__ double Fma(double a, double b, double c) { return fma(a, b, c); }
+__device__ __forceinline__ double Mul(double a, double b) { return a*b; }
+
+template <class V> struct Two {
+	V a, b;
+};
+
+// G_0 .. G_3 of row field I and column field F.  coef(k): number k of the point, coef.two(k): numbers k and
+// k + 1 (k even); g: gradient of N_b, l: L.  V: double, or a packed pair of floats with its own Fma and Mul.
 template <int I, int F, class V, class Coef>
 __device__ __forceinline__ void TangentColumn(const Coef& coef, V n, const V g[3], V l, V inverse_density, V out[4])
 {
 	if constexpr (I < 3 && F < 3) {
-		out[0] = coef(kPackNN+3*I+F)*n-coef(kPackTg+3*I+F)*l;
-		if constexpr (I == F)
-			out[0] = out[0]+coef(kPackRa)*g[0]+coef(kPackRa+1)*g[1]+coef(kPackRa+2)*g[2];
-		#pragma unroll
-		for (int d = 0; d < 3; ++d) {
-			V v = coef(kPackC+9*I+3*F+d)*n;
-			if (I == F) v = v+coef(kPackMu)*g[d]+coef(kPackPa+d)*l;
-			if (d == I) v = v+coef(kPackTauC)*g[F];
-			if (d == F) v = v+coef(kPackMu)*g[I]+coef(kPackPf+I)*l;
-			out[1+d] = v;
+		constexpr int kColumn = kPackColumn+6*(3*I+F);
+		const Two<V> nt = coef.two(kColumn), c01 = coef.two(kColumn+2), c2 = coef.two(kColumn+4);
+		const Two<V> pt = coef.two(kPackPa+2), rm = coef.two(kPackRa+2);     // pa_2, tau_C; ra_2, mu
+		const V c[3] = {c01.a, c01.b, c2.a}, pf = coef(kPackPf+I);
+		out[0] = Fma(nt.a, n, Mul(nt.b, l));
+		if constexpr (I == F) {
+			const Two<V> ra = coef.two(kPackRa), pa = coef.two(kPackPa);
+			const V p[3] = {pa.a, pa.b, pt.a};
+			out[0] = Fma(ra.a, g[0], Fma(ra.b, g[1], Fma(rm.a, g[2], out[0])));
+			#pragma unroll
+			for (int d = 0; d < 3; ++d) out[1+d] = Fma(rm.b, g[d], Fma(p[d], l, Mul(c[d], n)));
+			out[1+I] = Fma(pt.b, g[I], Fma(rm.b, g[I], Fma(pf, l, out[1+I])));
+		} else {
+			#pragma unroll
+			for (int d = 0; d < 3; ++d) out[1+d] = Mul(c[d], n);
+			out[1+I] = Fma(pt.b, g[F], out[1+I]);
+			out[1+F] = Fma(rm.b, g[I], Fma(pf, l, out[1+F]));
 		}
 	} else if constexpr (I < 3) {
-		const V t = coef(kPackTg+3*I)*g[0]+coef(kPackTg+3*I+1)*g[1]+coef(kPackTg+3*I+2)*g[2];
-		out[0] = -inverse_density*t;
+		const V pf = coef(kPackPf+I);
+		const Two<V> pa = coef.two(kPackPa);
+		const V p[3] = {pa.a, pa.b, coef(kPackPa+2)};
+		out[0] = Mul(inverse_density, Fma(coef(kPackColumn+18*I+1), g[0],
+			Fma(coef(kPackColumn+18*I+7), g[1], Mul(coef(kPackColumn+18*I+13), g[2]))));
 		#pragma unroll
 		for (int d = 0; d < 3; ++d) {
-			V v = inverse_density*(coef(kPackPa+d)*g[I]+coef(kPackPf+I)*g[d]);
-			if (d == I) v = v-coef(kPackOne)*n;
-			out[1+d] = v;
+			const V w = Fma(p[d], g[I], Mul(pf, g[d]));
+			out[1+d] = d == I ? Fma(inverse_density, w, Mul(coef(kPackMinusOne), n)) : Mul(inverse_density, w);
 		}
 	} else if constexpr (F < 3) {
-		out[0] = coef(kPackOne)*g[F];
+		out[0] = Mul(coef(kPackOne), g[F]);
 		#pragma unroll
 		for (int d = 0; d < 3; ++d) {
-			V v = -coef(kPackA+3*d+F)*n;
-			if (d == F) v = v+coef(kPackTau)*l;
-			out[1+d] = v;
+			const V w = Mul(coef(kPackColumn+6*(3*d+F)+5), n);
+			out[1+d] = d == F ? Fma(coef(kPackTau), l, w) : w;
 		}
 	} else {
-		out[0] = V(0);
+		const V t = coef(kPackTauRho);
+		out[0] = V{};
 		#pragma unroll
-		for (int d = 0; d < 3; ++d) out[1+d] = coef(kPackTauRho)*g[d];
+		for (int d = 0; d < 3; ++d) out[1+d] = Mul(t, g[d]);
 	}
 }
 
