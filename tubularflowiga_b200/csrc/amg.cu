@@ -986,12 +986,9 @@ AmgResidentView Amg::ResidentView()
 	AmgResidentView v;
 	v.coarse = C.nodes;
 	v.agg = L.agg.get();
-	v.agg_order = L.agg_order.get();
-	v.agg_offsets = L.agg_offsets.get();
 	v.mask = L.mask.get();
 	v.dense = C.dense_inverse;
 	v.dense_ld = C.dense_ld;
-	v.coarse_rhs = C.b.get();
 	v.coarse_x = C.x.get();
 	v.ap_rows = L.ap_rows.get();
 	v.ap_cols = L.ap_cols.get();

@@ -8,11 +8,15 @@
 // contiguous range of block rows, balanced by blocks, and keeps its slice of the whole basis in shared
 // memory, so both Gram-Schmidt passes read no memory beyond the partial sums; its work vector, the
 // rotations and the Hessenberg column live there too.  A step then costs its SpMV, the AMG arrays and
-// six grid barriers (three without AMG) of about 1.2 us.
+// five grid barriers (three without AMG) of 1.7 us.  Measured per step, separate launches against this kernel:
+// cylinder, block-Jacobi FP64 GMRES(200) 68 -> 23 us, AMG-FGMRES FP64 70 -> 29 us; 12,800-element section, AMG-FGMRES
+// FP32 105 -> 84 us (its 199 MB matrix streams from HBM), its transport GMRES(50) 58 -> 25 us; 6,176-element batch of
+// five tubes 92 -> 35 us.
 //
-// Phases of a step, a barrier after each: [restrict v_j | dense coarse solve | coarse correction and
-// block-Jacobi: z_j |] SpMV of the own rows and first-pass dots | update and second-pass dots | update,
-// v_{j+1} published, its norm.  Every CTA sums the others' partial sums itself in the same fixed order, so
+// Phases of a step, a barrier after each: [dense coarse solve | coarse correction and block-Jacobi: z_j |] SpMV of
+// the own rows and first-pass dots | update and second-pass dots | update, v_{j+1} published with its norm and, for
+// the coarse solve, every CTA's share of the aggregates' sums.  The rotations of a step run beside the next
+// step's first phase.  Every CTA sums the others' partial sums itself in the same fixed order, so
 // all of them take the same decisions without a broadcast, and results do not depend on timing.
 //
 // Independent segments (a batch of tubes) are groups of CTAs: each group has its own coefficients, norms,
@@ -31,20 +35,31 @@
 namespace tfiga {
 namespace {
 
-constexpr int kThreads = 1024;
-constexpr int kWarps = kThreads/32;
+// Threads per CTA: the flexible solves carry the AMG phases and gain from 128 registers (section step 51.9 ms in this
+// kernel with 1024 threads, 47.3 with 512); the left-preconditioned ones spend most of a step on the Gram-Schmidt
+// passes and gain from twice the threads (cylinder block-Jacobi solve 10.1 ms with 512, 9.4 with 1024).
+constexpr int kThreadsFlexible = 512, kThreadsLeft = 1024;
 constexpr int kMaxRestart = 256;
 constexpr int kMaxPieces = 4;
-constexpr int kRestrictWarps = 8;              // warps per aggregate
 constexpr int kDenseRows = 64;                 // coarse rows per CTA at most
+constexpr int kCoarseMax = 512;                // aggregates at most (a coarse vector in shared memory)
+// A matrix of at most this many bytes stays in the L2 (126 MB) from one product to the next, beside the vectors and the
+// AMG's arrays; a larger one is loaded to leave the L2 first, so that the vectors stay.  (82 MB batch: 3.65 ms a solve
+// streamed, 3.12 ms kept; 199 MB section: 7.75 ms streamed, 8.2 to 8.6 ms with 48 to 96 MB of it kept.)
+constexpr size_t kKeepBytes = (size_t)96 << 20;
 constexpr unsigned long long kWaitNs = 4000000000ull;
 constexpr int kIterationsPerLaunch = 4096;     // bounds one launch; a longer solve continues in the next
 
 struct Args {
 	ResidentProblem p;
 	int restart, slice, pieces, ctas, groups;
+	bool keep;                                 // the matrix stays in the L2
 	int max_cycles_iterations;
 	const int32_t *cta_row, *cta_group, *group_cta, *agg_list, *agg_list_offsets;
+	// restriction: the nodes of every CTA by aggregate (part_nodes from part_start of its parts cta_parts ..), a
+	// partial sum per part; each aggregate's parts are part_list from part_offsets; aggregates by group
+	const int32_t *cta_parts, *part_start, *part_nodes, *part_offsets, *part_list, *group_agg, *group_agg_offsets;
+	double* coarse_part;
 	double *partial, *R, *y;
 	const double* tolerance_in;                // a continued solve's tolerances, else null
 	double* tolerance_out;
@@ -94,80 +109,87 @@ __device__ __forceinline__ double2 Load2(const double* p)
 	return v;
 }
 
-// Lane's part of block row `row`, blocks first, first + step, ...: for 4x4 blocks four lanes share a
-// block, one row each (a warp reads eight consecutive blocks at once, contiguously), so a row's sum needs
-// three shuffles; for 2x2 blocks a lane takes a whole block.
-template <int F, class T> struct RowPiece;
-
+// 4x4 blocks: four lanes share a block, one row each (a warp reads eight consecutive blocks at once, contiguously), so
+// a row's sum needs three shuffles; 2x2 blocks: a lane takes a whole block.
+template <bool kStream, class V> __device__ __forceinline__ V LoadMatrix(const V* p)
+{
+	if constexpr (kStream) return __ldcs(p);
+	else return __ldg(p);
+}
 template <class T> struct BlockRow;
 template <> struct BlockRow<float> {
-	static __device__ __forceinline__ void Get(const float* v, size_t block, int r, double a[4])
+	float4 q;
+	template <bool kStream> __device__ __forceinline__ void Load(const float* v, size_t block, int r)
 	{
-		const float4 q = __ldcs(reinterpret_cast<const float4*>(v+block*16+4*r));
-		a[0] = q.x; a[1] = q.y; a[2] = q.z; a[3] = q.w;
+		q = LoadMatrix<kStream>(reinterpret_cast<const float4*>(v+block*16+4*r));
+	}
+	__device__ __forceinline__ double Dot(double2 x, double2 y, double s) const
+	{
+		s = fma((double)q.x, x.x, s); s = fma((double)q.y, x.y, s);
+		return fma((double)q.w, y.y, fma((double)q.z, y.x, s));
 	}
 };
 template <> struct BlockRow<double> {
-	static __device__ __forceinline__ void Get(const double* v, size_t block, int r, double a[4])
+	double2 a, b;
+	template <bool kStream> __device__ __forceinline__ void Load(const double* v, size_t block, int r)
 	{
 		const double2* q = reinterpret_cast<const double2*>(v+block*16+4*r);
-		const double2 x = __ldg(q), y = __ldg(q+1);
-		a[0] = x.x; a[1] = x.y; a[2] = y.x; a[3] = y.y;
+		a = LoadMatrix<kStream>(q);
+		b = LoadMatrix<kStream>(q+1);
+	}
+	__device__ __forceinline__ double Dot(double2 x, double2 y, double s) const
+	{
+		s = fma(a.x, x.x, s); s = fma(a.y, x.y, s);
+		return fma(b.y, y.y, fma(b.x, y.x, s));
 	}
 };
 
-template <class T> struct RowPiece<4, T> {
-	// the row sum r in lane r = 0 .. 3
-	static __device__ __forceinline__ void Sum(const T* values, const int32_t* cols, const double* x, int lo, int hi,
-		int lane, double out[1])
-	{
+__device__ __forceinline__ double QuadRowSum(double s)     // the row sum r in lanes with lane & 3 == r
+{
+	#pragma unroll
+	for (int o = 16; o >= 4; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+	return s;
+}
+
+// One piece of a block row, blocks lo .. hi - 1: the row sum r in lane r < F.
+template <int F, class T, bool kStream>
+__device__ __forceinline__ double PieceSum(const T* values, const int32_t* cols, const double* x, int lo, int hi,
+	int lane)
+{
+	if constexpr (F == 4) {
 		constexpr int kUnroll = sizeof(T) == 4 ? 4 : 2;
 		const int r = lane & 3;
 		double s = 0.0;
 		int b = lo+(lane >> 2);
 		for (; b+8*(kUnroll-1) < hi; b += 8*kUnroll) {
 			int c[kUnroll];
-			double a[kUnroll][4];
+			BlockRow<T> a[kUnroll];
 			#pragma unroll
 			for (int u = 0; u < kUnroll; ++u) c[u] = __ldg(cols+b+8*u);
 			#pragma unroll
-			for (int u = 0; u < kUnroll; ++u) BlockRow<T>::Get(values, (size_t)(b+8*u), r, a[u]);
+			for (int u = 0; u < kUnroll; ++u) a[u].template Load<kStream>(values, (size_t)(b+8*u), r);
 			#pragma unroll
-			for (int u = 0; u < kUnroll; ++u) {
-				const double2 p = Load2(x+4*(size_t)c[u]), q = Load2(x+4*(size_t)c[u]+2);
-				s = fma(a[u][0], p.x, s); s = fma(a[u][1], p.y, s);
-				s = fma(a[u][2], q.x, s); s = fma(a[u][3], q.y, s);
-			}
+			for (int u = 0; u < kUnroll; ++u) s = a[u].Dot(Load2(x+4*(size_t)c[u]), Load2(x+4*(size_t)c[u]+2), s);
 		}
 		for (; b < hi; b += 8) {
 			const int c = __ldg(cols+b);
-			double a[4];
-			BlockRow<T>::Get(values, (size_t)b, r, a);
-			const double2 p = Load2(x+4*(size_t)c), q = Load2(x+4*(size_t)c+2);
-			s = fma(a[0], p.x, s); s = fma(a[1], p.y, s); s = fma(a[2], q.x, s); s = fma(a[3], q.y, s);
+			BlockRow<T> a;
+			a.template Load<kStream>(values, (size_t)b, r);
+			s = a.Dot(Load2(x+4*(size_t)c), Load2(x+4*(size_t)c+2), s);
 		}
-		#pragma unroll
-		for (int o = 16; o >= 4; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-		out[0] = s;
-	}
-};
-
-template <class T> struct RowPiece<2, T> {
-	// the row sum r in lane r = 0, 1
-	static __device__ __forceinline__ void Sum(const T* values, const int32_t* cols, const double* x, int lo, int hi,
-		int lane, double out[1])
-	{
+		return QuadRowSum(s);
+	} else {
 		double s0 = 0.0, s1 = 0.0;
 		#pragma unroll 2
 		for (int b = lo+lane; b < hi; b += 32) {
 			const int c = __ldg(cols+b);
 			double a[4];
 			if constexpr (sizeof(T) == 4) {
-				const float4 q = __ldg(reinterpret_cast<const float4*>(values+4*(size_t)b));
+				const float4 q = LoadMatrix<kStream>(reinterpret_cast<const float4*>(values+4*(size_t)b));
 				a[0] = q.x; a[1] = q.y; a[2] = q.z; a[3] = q.w;
 			} else {
 				const double2* q = reinterpret_cast<const double2*>(values+4*(size_t)b);
-				const double2 u = __ldg(q), v = __ldg(q+1);
+				const double2 u = LoadMatrix<kStream>(q), v = LoadMatrix<kStream>(q+1);
 				a[0] = u.x; a[1] = u.y; a[2] = v.x; a[3] = v.y;
 			}
 			const double2 v = Load2(x+2*(size_t)c);
@@ -179,21 +201,25 @@ template <class T> struct RowPiece<2, T> {
 		keep += __shfl_xor_sync(0xffffffffu, give, 1);
 		#pragma unroll
 		for (int o = 16; o >= 2; o >>= 1) keep += __shfl_xor_sync(0xffffffffu, keep, o);
-		out[0] = keep;
+		return keep;
 	}
-};
+}
 
 template <class B> __device__ __forceinline__ double BasisLoad(const B* p)
 {
 	return (double)*reinterpret_cast<const volatile B*>(p);
 }
 
+// Doubles that the own rows' offsets take (even, so that what follows stays 16-byte aligned).
+__host__ __device__ constexpr int RowSlots(int slice, int fields) { return ((slice/fields+2)/2+2) & ~1; }
+
 template <int F, class T, class RT, class B, bool kFlex>
-__global__ void __launch_bounds__(kThreads, 1) ResidentKrylovKernel(const Args a)
+__global__ void __launch_bounds__(kFlex ? kThreadsFlexible : kThreadsLeft, 1) ResidentKrylovKernel(const Args a)
 {
+	constexpr int kThreads = kFlex ? kThreadsFlexible : kThreadsLeft, kWarps = kThreads/32;
 	extern __shared__ __align__(16) double sm[];
-	__shared__ double red[kWarps][4];
-	__shared__ double dense_part[kDenseRows][8];
+	__shared__ double red[kWarps];
+	__shared__ double dense_part[kFlex ? kDenseRows : 1][8];
 	__shared__ double low_dot;
 	__shared__ int expired;
 	__shared__ double s_next;
@@ -201,7 +227,7 @@ __global__ void __launch_bounds__(kThreads, 1) ResidentKrylovKernel(const Args a
 	const int m1 = a.restart+1;
 	double* w = sm;                                    // [slice] work vector
 	double* piece = w+a.slice;                         // [pieces * slice] SpMV pieces
-	double* part = piece+(size_t)a.pieces*a.slice;     // [1024] update parts
+	double* part = piece+(size_t)a.pieces*a.slice;     // [kThreads] update parts
 	double* h = part+kThreads;                         // [restart + 1] this pass's coefficients
 	double* col = h+m1;                                // [restart + 1] Hessenberg column
 	double* scale = col+m1;
@@ -210,7 +236,9 @@ __global__ void __launch_bounds__(kThreads, 1) ResidentKrylovKernel(const Args a
 	double* g = sn+m1;
 	double* pc = g+m1;                                 // rotation products
 	double* tt = pc+m1;                                // rotation carries
-	B* Vs = reinterpret_cast<B*>(tt+m1+(m1 & 1));      // [restart + 1][slice]
+	int* rows = reinterpret_cast<int*>(tt+m1);          // [slice / F + 1] own row offsets
+	double* coarse_b = tt+m1+RowSlots(a.slice, F);      // [4 coarse] the group's restricted vector (flexible)
+	B* Vs = reinterpret_cast<B*>(coarse_b+(kFlex ? 4*kCoarseMax : 0));   // [restart + 1][slice]
 
 	const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
 	const int cta = blockIdx.x, G = a.ctas;
@@ -227,20 +255,29 @@ __global__ void __launch_bounds__(kThreads, 1) ResidentKrylovKernel(const Args a
 	double* norms = a.partial+(size_t)2*G*m1;
 	unsigned epoch = 0;
 	if (tid == 0) expired = 0;
+	for (int r = tid; r <= row1-row0; r += kThreads) rows[r] = a.p.pattern.row_offsets[row0+r];
+	__syncthreads();
 	auto barrier = [&]() { ++epoch; return GridBarrier(a.barrier, epoch*(unsigned)G, &expired); };
 
-	// Own rows of A v into `piece`, one warp per (row, piece of its blocks).
-	auto product = [&](const auto* values, const double* x) {
+	// Own rows of A x into `piece`, one warp per (row, piece of its blocks); warps `skip` and up take part.
+	auto product = [&](const auto* values, const double* x, int skip, bool keep) {
 		using VT = std::remove_cv_t<std::remove_pointer_t<decltype(values)>>;
-		const int P = a.pieces, rows = row1-row0;
-		for (int t = warp; t < rows*P; t += kWarps) {
+		if (warp < skip) return;
+		const int P = a.pieces, tasks = (row1-row0)*P, stride = kWarps-skip;
+		const auto bounds = [&](int t, int& lo_, int& hi_) {
 			const int r = t/P, q = t-r*P;
-			const int b0 = a.p.pattern.row_offsets[row0+r], b1 = a.p.pattern.row_offsets[row0+r+1];
+			const int b0 = rows[r], b1 = rows[r+1];
 			const int per = (b1-b0+P-1)/P;
-			const int s0 = min(b1, b0+q*per), s1 = min(b1, s0+per);
-			double v[1];
-			RowPiece<F, VT>::Sum(values, a.p.pattern.columns, x, s0, s1, lane, v);
-			if (lane < F) piece[(size_t)q*a.slice+F*r+lane] = v[0];
+			lo_ = min(b1, b0+q*per);
+			hi_ = min(b1, lo_+per);
+		};
+		for (int t = warp-skip; t < tasks; t += stride) {
+			int b0, b1;
+			bounds(t, b0, b1);
+			const double v = keep
+				? PieceSum<F, VT, false>(values, a.p.pattern.columns, x, b0, b1, lane)
+				: PieceSum<F, VT, true>(values, a.p.pattern.columns, x, b0, b1, lane);
+			if (lane < F) piece[(size_t)(t%P)*a.slice+F*(t/P)+lane] = v;
 		}
 	};
 	auto piece_sum = [&](int k) {
@@ -258,10 +295,10 @@ __global__ void __launch_bounds__(kThreads, 1) ResidentKrylovKernel(const Args a
 			for (int e = e0+tid; e < e1; e += kThreads)
 				s = fma(a.p.low.val[e], *reinterpret_cast<const volatile double*>(x+a.p.low.idx[e]), s);
 			s = WarpSum(s);
-			if (lane == 0) red[warp][0] = s;
+			if (lane == 0) red[warp] = s;
 			__syncthreads();
 			if (warp == 0) {
-				const double t = WarpSum(red[lane][0]);
+				const double t = WarpSum(lane < kWarps ? red[lane] : 0.0);
 				if (lane == 0) low_dot = a.p.low.coef[k]*t;
 			}
 			__syncthreads();
@@ -311,24 +348,27 @@ __global__ void __launch_bounds__(kThreads, 1) ResidentKrylovKernel(const Args a
 			if (sl == 0 && i < count) out[(size_t)i*G+cta] = s*scale[i];
 		}
 	};
-	// h_i = sum of the group's partial sums; the column accumulates over the passes.
+	// h_i = sum of the group's partial sums (several basis vectors per warp at a time, their loads in flight
+	// together); the column accumulates over the passes.
 	auto gather_dots = [&](int count, const double* in, bool first) {
-		for (int i = warp; i < count; i += 2*kWarps) {
-			const int i2 = i+kWarps;
-			const bool two = i2 < count;
-			double s = 0.0, t = 0.0;
-			for (int c = g0+lane; c < g1; c += 32) {
-				s += *reinterpret_cast<const volatile double*>(in+(size_t)i*G+c);
-				if (two) t += *reinterpret_cast<const volatile double*>(in+(size_t)i2*G+c);
-			}
-			s = WarpSum(s);
-			t = WarpSum(t);
-			if (lane == 0) {
-				h[i] = s*scale[i];
-				col[i] = first ? s : col[i]+s;
-				if (two) {
-					h[i2] = t*scale[i2];
-					col[i2] = first ? t : col[i2]+t;
+		constexpr int kAtOnce = kFlex ? 4 : 2;
+		for (int i = warp; i < count; i += kAtOnce*kWarps) {
+			double s[kAtOnce];
+			#pragma unroll
+			for (int u = 0; u < kAtOnce; ++u) s[u] = 0.0;
+			for (int c = g0+lane; c < g1; c += 32)
+				#pragma unroll
+				for (int u = 0; u < kAtOnce; ++u)
+					if (i+u*kWarps < count)
+						s[u] += *reinterpret_cast<const volatile double*>(in+(size_t)(i+u*kWarps)*G+c);
+			#pragma unroll
+			for (int u = 0; u < kAtOnce; ++u) {
+				const int k = i+u*kWarps;
+				if (k >= count) break;
+				const double v = WarpSum(s[u]);
+				if (lane == 0) {
+					h[k] = v*scale[k];
+					col[k] = first ? v : col[k]+v;
 				}
 			}
 		}
@@ -380,11 +420,24 @@ __global__ void __launch_bounds__(kThreads, 1) ResidentKrylovKernel(const Args a
 			sq = fma(v, v, sq);
 		}
 		sq = WarpSum(sq);
-		if (lane == 0) red[warp][0] = sq;
+		if (lane == 0) red[warp] = sq;
 		__syncthreads();
 		if (warp == 0) {
-			sq = WarpSum(red[lane][0]);
+			sq = WarpSum(lane < kWarps ? red[lane] : 0.0);
 			if (lane == 0) norms[cta] = sq;
+		}
+		if constexpr (kFlex) {
+			// the vector's share of every aggregate with nodes here: a warp per part, four lanes (fields) per node
+			for (int k = a.cta_parts[cta]+warp; k < a.cta_parts[cta+1]; k += kWarps) {
+				const int e1 = a.part_start[k+1];
+				double s = 0.0;
+				for (int e = a.part_start[k]+(lane >> 2); e < e1; e += 8) {
+					const int i = 4*a.part_nodes[e]+(lane & 3);
+					s = fma(a.p.amg.mask[i], (double)Vs[(size_t)j*a.slice+i-lo], s);
+				}
+				s = QuadRowSum(s);
+				if (lane < 4) a.coarse_part[4*(size_t)k+lane] = s;
+			}
 		}
 	};
 	auto group_norm = [&](int from, int to) {           // one warp; every lane gets the norm
@@ -394,7 +447,8 @@ __global__ void __launch_bounds__(kThreads, 1) ResidentKrylovKernel(const Args a
 	};
 	// w = [D^-1] (rhs - A x) of the own rows
 	auto residual = [&]() {
-		product(static_cast<const RT*>(a.p.residual_values), a.p.x);
+		product(static_cast<const RT*>(a.p.residual_values), a.p.x, 0,
+			a.keep && a.p.residual_values == a.p.krylov_values);
 		__syncthreads();
 		if (kFlex && a.p.low.count) low_rank(a.p.x);
 		for (int k = tid; k < len; k += kThreads) w[k] = a.p.rhs[lo+k]-piece_sum(k);
@@ -481,44 +535,98 @@ __global__ void __launch_bounds__(kThreads, 1) ResidentKrylovKernel(const Args a
 			if (leader) a.flags[grp] = open ? 0 : 1;
 		}
 		__syncthreads();
+		// rotations of column j, by one warp: t_{i+1} = -s_i t_i + c_i h_{i+1} is the only serial part
+		auto rotate = [&](int j) {
+			const double next = group_norm(g0, g1);
+			if (lane == 0) col[j+1] = next;
+			__syncwarp();
+			for (int i = lane; i < j; i += 32) pc[i] = cs[i]*col[i+1];
+			__syncwarp();
+			if (lane == 0) {
+				double t = col[0];
+				#pragma unroll 8
+				for (int i = 0; i < j; ++i) { tt[i] = t; t = fma(-sn[i], t, pc[i]); }
+				const double mag = hypot(t, next);
+				const double c = mag > 0.0 ? t/mag : 1.0, s = mag > 0.0 ? next/mag : 0.0;
+				cs[j] = c; sn[j] = s;
+				const double old = g[j];
+				g[j] = c*old;
+				g[j+1] = -s*old;
+				const double res = fabs(g[j+1]);
+				const int stop = res <= tolerance || next <= 1e-30;
+				scale[j+1] = next > 1e-30 && !(stop && a.groups > 1) ? 1.0/next : 0.0;
+				s_stop = stop;
+				if (leader) {
+					R[(size_t)j*m1+j] = mag;
+					if (stop) a.flags[grp] = 1;
+				}
+			}
+			__syncwarp();
+			if (leader)
+				for (int i = lane; i < j; i += 32) R[(size_t)j*m1+i] = fma(cs[i], tt[i], sn[i]*col[i+1]);
+		};
+		// Step j: the rotations of step j - 1 run in warp 0 beside the next thing that does not need them (the
+		// coarse solve of the unscaled v_j, or its product); a stop discards that.
 		int used = 0, j = 0;
-		for (; j < cap; ++j) {
+		for (;; ++j) {
+			const bool rotating = j > 0 && open;
+			if (rotating && warp == 0) rotate(j-1);
 			if constexpr (kFlex) {
-				// restriction of v_j: eight warps per aggregate of this CTA's list
-				const int slots = kWarps/kRestrictWarps, slot = warp/kRestrictWarps;
-				const int a0 = a.agg_list_offsets[cta], a1 = a.agg_list_offsets[cta+1];
-				for (int base = a0; base < a1; base += slots) {
-					const int which = base+slot;
-					double acc[4] = {0.0, 0.0, 0.0, 0.0};
-					if (which < a1 && open) {
-						const int I = a.agg_list[which];
-						const double s = scale[j];
-						const int e1 = a.p.amg.agg_offsets[I+1];
-						for (int k = a.p.amg.agg_offsets[I]+(tid & (32*kRestrictWarps-1)); k < e1; k += 32*kRestrictWarps) {
-							const size_t i = 4*(size_t)a.p.amg.agg_order[k];
-							const double2 m01 = *reinterpret_cast<const double2*>(a.p.amg.mask+i);
-							const double2 m23 = *reinterpret_cast<const double2*>(a.p.amg.mask+i+2);
-							const B* v = V+(size_t)j*n+i;
-							acc[0] += m01.x*(s*BasisLoad(v)); acc[1] += m01.y*(s*BasisLoad(v+1));
-							acc[2] += m23.x*(s*BasisLoad(v+2)); acc[3] += m23.y*(s*BasisLoad(v+3));
-						}
+				// the group's restricted v_j (unscaled) into shared memory: four threads per aggregate
+				const int q0 = a.group_agg_offsets[grp], q1 = a.group_agg_offsets[grp+1];
+				const int from = rotating ? 32 : 0;
+				if (j < cap && tid >= from)
+					for (int k = tid-from; k < 4*(q1-q0); k += kThreads-from) {
+						const int I = a.group_agg[q0+(k >> 2)];
+						const int e1 = a.part_offsets[I+1];
+						double s = 0.0;
+						#pragma unroll 4
+						for (int e = a.part_offsets[I]; e < e1; ++e)
+							s += *reinterpret_cast<const volatile double*>(a.coarse_part+4*(size_t)a.part_list[e]+(k & 3));
+						coarse_b[k] = s;
 					}
-					#pragma unroll
-					for (int c = 0; c < 4; ++c) {
-						acc[c] = WarpSum(acc[c]);
-						if (lane == 0) red[warp][c] = acc[c];
+			} else {
+				if (j < cap)
+					product(static_cast<const T*>(a.p.krylov_values), reinterpret_cast<const double*>(V)+(size_t)j*n,
+						rotating ? 1 : 0, a.keep);
+			}
+			__syncthreads();
+			if (rotating) {
+				used = j;
+				if (s_stop) {
+					open = false;
+					if (a.groups == 1) break;
+				}
+			}
+			if (j == cap) break;
+			if constexpr (kFlex) {
+				// dense coarse solve: the rows of this CTA's aggregates, each by `split` warps, over the group's columns
+				const int l0 = a.agg_list_offsets[cta], mine = 4*(a.agg_list_offsets[cta+1]-l0);
+				const int q0 = a.group_agg_offsets[grp], n2 = 2*(a.group_agg_offsets[grp+1]-q0);
+				if (open) {
+					int split = 1;
+					while (split < 8 && 2*split*mine <= kWarps && 32*split < n2) split *= 2;
+					for (int t = warp; t < mine*split; t += kWarps) {
+						const int k = t/split, q = t-k*split;
+						const double2* ar = reinterpret_cast<const double2*>(
+							a.p.amg.dense+(size_t)(4*a.agg_list[l0+(k >> 2)]+(k & 3))*a.p.amg.dense_ld);
+						double s = 0.0, u = 0.0;
+						#pragma unroll 4
+						for (int c = q*32+lane; c < n2; c += 32*split) {
+							const double2 e = __ldg(ar+2*__ldg(a.group_agg+q0+(c >> 1))+(c & 1));
+							const double2 b = *reinterpret_cast<const double2*>(coarse_b+2*c);
+							s = fma(e.x, b.x, s);
+							u = fma(e.y, b.y, u);
+						}
+						s = WarpSum(s+u);
+						if (lane == 0) dense_part[k][q] = s;
 					}
 					__syncthreads();
-					if (tid < 4*slots) {
-						const int q = base+tid/4;
-						if (q < a1) {
-							double s = 0.0;
-							#pragma unroll
-							for (int u = 0; u < kRestrictWarps; ++u) s += red[(tid/4)*kRestrictWarps+u][tid & 3];
-							a.p.amg.coarse_rhs[4*(size_t)a.agg_list[q]+(tid & 3)] = s;
-						}
+					if (tid < mine) {
+						double s = dense_part[tid][0];
+						for (int q = 1; q < split; ++q) s += dense_part[tid][q];
+						a.p.amg.coarse_x[4*(size_t)a.agg_list[l0+(tid >> 2)]+(tid & 3)] = s*scale[j];
 					}
-					__syncthreads();
 				}
 				if (!barrier()) return give_up(iterations);
 				if (a.groups > 1) {
@@ -533,74 +641,63 @@ __global__ void __launch_bounds__(kThreads, 1) ResidentKrylovKernel(const Args a
 					__syncthreads();
 					if (s_all) break;
 				}
-				// dense coarse solve: rows cta, cta + G, ..., each by `split` warps
-				const int dn = 4*a.p.amg.coarse;
-				const int mine = (dn-cta+G-1)/G;
-				int split = 1;
-				while (split < 8 && 2*split*mine <= kWarps && 64*split < dn) split *= 2;
-				for (int t = warp; t < mine*split; t += kWarps) {
-					const int k = t/split, q = t-k*split;
-					const double2* ar = reinterpret_cast<const double2*>(a.p.amg.dense+(size_t)(cta+G*k)*a.p.amg.dense_ld);
-					const int n2 = dn/2;
-					double s = 0.0, u = 0.0;
-					#pragma unroll 4
-					for (int c = q*32+lane; c < n2; c += 32*split) {
-						const double2 e = __ldg(ar+c), b = Load2(a.p.amg.coarse_rhs+2*c);
-						s = fma(e.x, b.x, s);
-						u = fma(e.y, b.y, u);
-					}
-					s = WarpSum(s+u);
-					if (lane == 0) dense_part[k][q] = s;
-				}
-				__syncthreads();
-				if (tid < mine) {
-					double s = dense_part[tid][0];
-					for (int q = 1; q < split; ++q) s += dense_part[tid][q];
-					a.p.amg.coarse_x[cta+G*tid] = s;
-				}
-				if (!barrier()) return give_up(iterations);
-				// z = P x_c + omega D^-1 (v - (A P) x_c), four lanes per node
+				// z = P x_c + omega D^-1 (v - (A P) x_c), `lanes` per node (four rows, the A P blocks split over the
+				// rest), x_c from shared memory
 				double* z = a.p.Z+(size_t)j*n;
 				if (open) {
+					for (int k = tid; k < 2*a.p.amg.coarse; k += kThreads)
+						reinterpret_cast<double2*>(coarse_b)[k] = Load2(a.p.amg.coarse_x+2*k);
+					__syncthreads();
 					const T* ap = static_cast<const T*>(a.p.amg.ap);
 					const double s = scale[j];
-					for (int k = tid; k < (len+31)/32*32; k += kThreads) {
-						const int i = row0+(k >> 2), r = k & 3;
-						const bool live = k < len;
+					int lanes = 4;
+					while (lanes < 32 && 2*lanes*(row1-row0) <= kThreads) lanes *= 2;
+					const int r = lane & 3, sub = (lane%lanes) >> 2, step = lanes >> 2;
+					for (int k = tid; k < ((row1-row0)*lanes+31)/32*32; k += kThreads) {
+						const int node = k/lanes, i = row0+node;
+						const bool live = node < row1-row0;
 						double v = 0.0;
 						if (live) {
-							v = s*(double)Vs[(size_t)j*a.slice+k];
 							const int e1 = a.p.amg.ap_rows[i+1];
-							for (int e = a.p.amg.ap_rows[i]; e < e1; ++e) {
-								double b[4];
-								BlockRow<T>::Get(ap, (size_t)e, r, b);
-								const double* xc = a.p.amg.coarse_x+4*(size_t)a.p.amg.ap_cols[e];
-								const double2 p = Load2(xc), q = Load2(xc+2);
-								v -= b[0]*p.x+b[1]*p.y+b[2]*q.x+b[3]*q.y;
+							constexpr int kAtOnce = 4;
+							for (int e = a.p.amg.ap_rows[i]+sub; e < e1; e += kAtOnce*step) {
+								BlockRow<T> b[kAtOnce];
+								int c[kAtOnce];
+								#pragma unroll
+								for (int u = 0; u < kAtOnce; ++u) {
+									const int at = min(e+u*step, e1-1);
+									c[u] = __ldg(a.p.amg.ap_cols+at);
+									b[u].template Load<false>(ap, (size_t)at, r);
+								}
+								#pragma unroll
+								for (int u = 0; u < kAtOnce; ++u) {
+									const double2* xc = reinterpret_cast<const double2*>(coarse_b+4*c[u]);
+									if (e+u*step < e1) v -= b[u].Dot(xc[0], xc[1], 0.0);
+								}
 							}
 						}
+						for (int o = lanes >> 1; o >= 4; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+						if (live) v = fma(s, (double)Vs[(size_t)j*a.slice+4*node+r], v);
 						const int base = lane & ~3;
 						const double v0 = __shfl_sync(0xffffffffu, v, base), v1 = __shfl_sync(0xffffffffu, v, base+1);
 						const double v2 = __shfl_sync(0xffffffffu, v, base+2), v3 = __shfl_sync(0xffffffffu, v, base+3);
-						if (live) {
+						if (live && sub == 0) {
 							const double2* d = reinterpret_cast<const double2*>(a.p.amg.inverse+(size_t)i*16+4*r);
 							const double2 d01 = d[0], d23 = d[1];
-							const double xc = *reinterpret_cast<const volatile double*>(
-								a.p.amg.coarse_x+4*(size_t)a.p.amg.agg[i]+r);
-							z[lo+k] = a.p.amg.mask[lo+k]*xc+a.p.amg.omega*(d01.x*v0+d01.y*v1+d23.x*v2+d23.y*v3);
+							const size_t at = 4*(size_t)i+r;
+							z[at] = a.p.amg.mask[at]*coarse_b[4*a.p.amg.agg[i]+r]
+								+a.p.amg.omega*(d01.x*v0+d01.y*v1+d23.x*v2+d23.y*v3);
 						}
 					}
 				}
 				if (!barrier()) return give_up(iterations);
 				if (open) {
-					product(static_cast<const T*>(a.p.krylov_values), z);
+					product(static_cast<const T*>(a.p.krylov_values), z, 0, a.keep);
 					__syncthreads();
 					if (a.p.low.count) low_rank(z);
 					finish_product(1.0, false);
 				}
 			} else {
-				product(static_cast<const T*>(a.p.krylov_values), reinterpret_cast<const double*>(V)+(size_t)j*n);
-				__syncthreads();
 				finish_product(scale[j], true);
 			}
 			__syncthreads();
@@ -623,44 +720,6 @@ __global__ void __launch_bounds__(kThreads, 1) ResidentKrylovKernel(const Args a
 				publish(j+1);
 			}
 			if (!barrier()) return give_up(iterations);
-			if (open) {
-				if (warp == 0) {
-					// rotations of the new column: t_{i+1} = -s_i t_i + c_i h_{i+1} is the only serial part
-					const double next = group_norm(g0, g1);
-					if (lane == 0) col[j+1] = next;
-					__syncwarp();
-					for (int i = lane; i < j; i += 32) pc[i] = cs[i]*col[i+1];
-					__syncwarp();
-					if (lane == 0) {
-						double t = col[0];
-						#pragma unroll 8
-						for (int i = 0; i < j; ++i) { tt[i] = t; t = fma(-sn[i], t, pc[i]); }
-						const double mag = hypot(t, next);
-						const double c = mag > 0.0 ? t/mag : 1.0, s = mag > 0.0 ? next/mag : 0.0;
-						cs[j] = c; sn[j] = s;
-						const double old = g[j];
-						g[j] = c*old;
-						g[j+1] = -s*old;
-						const double res = fabs(g[j+1]);
-						const int stop = res <= tolerance || next <= 1e-30;
-						scale[j+1] = next > 1e-30 && !(stop && a.groups > 1) ? 1.0/next : 0.0;
-						s_stop = stop;
-						if (leader) {
-							R[(size_t)j*m1+j] = mag;
-							if (stop) a.flags[grp] = 1;
-						}
-					}
-					__syncwarp();
-					if (leader)
-						for (int i = lane; i < j; i += 32) R[(size_t)j*m1+i] = fma(cs[i], tt[i], sn[i]*col[i+1]);
-				}
-				__syncthreads();
-				used = j+1;
-				if (s_stop) {
-					open = false;
-					if (a.groups == 1) { ++j; break; }
-				}
-			}
 		}
 		iterations += j;
 		// least squares: back substitution by the leader's first warp, right-hand side in registers
@@ -753,6 +812,7 @@ bool ResidentKrylov::Prepare(Kind kind, const DevicePatternView& pattern, int re
 void ResidentKrylov::Plan(const DevicePatternView& pattern, const AmgResidentView* amg, cudaStream_t stream)
 {
 	const int fields = kind_ == kLeft2 || kind_ == kLeft2Fp32 ? 2 : 4;
+	threads_ = amg ? kThreadsFlexible : kThreadsLeft;
 	if (restart_ > kMaxRestart || pattern.nodes < 1) return;
 	int device = 0, sms = 0, cooperative = 0, shared_max = 0;
 	CudaCheck(cudaGetDevice(&device), "device");
@@ -806,20 +866,24 @@ void ResidentKrylov::Plan(const DevicePatternView& pattern, const AmgResidentVie
 		}
 		group_cta.push_back((int32_t)cta_group.size());
 	}
+	const size_t value_bytes = fields == 4 ? (kind_ == kLeft4 || kind_ == kFlexDouble ? 128 : 64)
+		: kind_ == kLeft2 ? 32 : 16;
+	keep_ = (size_t)blocks*value_bytes <= kKeepBytes;
 	int most_rows = 0;
 	for (int c = 0; c < ctas_; ++c) most_rows = std::max(most_rows, cta_row[c+1]-cta_row[c]);
 	// a slice stride of 8 modulo 16 entries spreads eight-lane dot groups over the banks
 	slice_ = (fields*most_rows+15)/16*16+8;
 	// split rows among warps until a CTA's last round of warps is a small part of its work
 	pieces_ = 1;
-	while (pieces_ < kMaxPieces && most_rows*pieces_ < 4*kWarps) pieces_ *= 2;
+	while (pieces_ < kMaxPieces && most_rows*pieces_ < threads_/8) pieces_ *= 2;
 	if (fields == 2) pieces_ = 1;
 	const size_t m1 = (size_t)restart_+1;
-	smem_ = ((size_t)slice_*(1+pieces_)+kThreads+8*m1+(m1 & 1))*sizeof(double)+m1*slice_*entry;
+	smem_ = ((size_t)slice_*(1+pieces_)+threads_+8*m1+RowSlots(slice_, fields)
+		+(amg ? 4*(size_t)kCoarseMax : 0))*sizeof(double)+m1*slice_*entry;
 	if (smem_+attributes.sharedSizeBytes > (size_t)shared_max) return;
+	if (groups_ > threads_) return;
 	if (amg) {
-		if (4*(long long)amg->coarse > (long long)ctas_*kDenseRows) return;
-		if (groups_ > kThreads) return;
+		if (amg->coarse > kCoarseMax) return;
 		// aggregates to CTAs of their own group, in turn
 		std::vector<int32_t> of((size_t)pattern.nodes);
 		CudaCheck(cudaMemcpyAsync(of.data(), amg->agg, of.size()*sizeof(int32_t), cudaMemcpyDeviceToHost, stream),
@@ -836,9 +900,44 @@ void ResidentKrylov::Plan(const DevicePatternView& pattern, const AmgResidentVie
 		}
 		std::vector<int32_t> list, offsets{0};
 		for (const auto& l : lists) {
+			if (4*l.size() > (size_t)kDenseRows) return;
 			list.insert(list.end(), l.begin(), l.end());
 			offsets.push_back((int32_t)list.size());
 		}
+		std::vector<int32_t> group_agg, group_agg_offsets{0};
+		for (int q = 0; q < groups_; ++q) {
+			for (int I = 0; I < amg->coarse; ++I)
+				if (group_of[I] == q) group_agg.push_back(I);
+			group_agg_offsets.push_back((int32_t)group_agg.size());
+		}
+		// every CTA's nodes by aggregate, and every aggregate's parts in the order of the CTAs
+		std::vector<int32_t> cta_parts{0}, part_start, part_nodes, part_agg;
+		for (int c = 0; c < ctas_; ++c) {
+			std::vector<int32_t> nodes(cta_row[c+1]-cta_row[c]);
+			for (size_t k = 0; k < nodes.size(); ++k) nodes[k] = cta_row[c]+(int32_t)k;
+			std::stable_sort(nodes.begin(), nodes.end(), [&](int32_t x, int32_t y) { return of[x] < of[y]; });
+			for (size_t k = 0; k < nodes.size(); ++k) {
+				if (k == 0 || of[nodes[k]] != of[nodes[k-1]]) {
+					part_start.push_back((int32_t)part_nodes.size());
+					part_agg.push_back(of[nodes[k]]);
+				}
+				part_nodes.push_back(nodes[k]);
+			}
+			cta_parts.push_back((int32_t)part_start.size());
+		}
+		part_start.push_back((int32_t)part_nodes.size());
+		std::vector<int32_t> part_offsets(amg->coarse+1, 0), part_list(part_agg.size());
+		for (const int32_t I : part_agg) ++part_offsets[I+1];
+		for (int I = 0; I < amg->coarse; ++I) part_offsets[I+1] += part_offsets[I];
+		std::vector<int32_t> fill(part_offsets.begin(), part_offsets.end()-1);
+		for (size_t k = 0; k < part_agg.size(); ++k) part_list[fill[part_agg[k]]++] = (int32_t)k;
+		const std::vector<int32_t>* tables[] = {&cta_parts, &part_start, &part_nodes, &part_offsets, &part_list, &group_agg,
+			&group_agg_offsets};
+		for (int k = 0; k < kTables; ++k) {
+			tables_[k].Allocate(tables[k]->size());
+			tables_[k].Upload(tables[k]->data(), tables[k]->size(), stream);
+		}
+		coarse_part_.Allocate(4*part_agg.size());
 		agg_list_.Allocate(list.size());
 		agg_list_.Upload(list.data(), list.size(), stream);
 		agg_list_offsets_.Allocate(offsets.size());
@@ -861,7 +960,7 @@ void ResidentKrylov::Plan(const DevicePatternView& pattern, const AmgResidentVie
 	CudaCheck(cudaFuncSetAttribute(reinterpret_cast<const void*>(kernel), cudaFuncAttributeMaxDynamicSharedMemorySize,
 		(int)(shared_max-attributes.sharedSizeBytes)), "resident GMRES shared memory");
 	int resident = 0;
-	CudaCheck(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, reinterpret_cast<const void*>(kernel), kThreads,
+	CudaCheck(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, reinterpret_cast<const void*>(kernel), threads_,
 		smem_), "resident GMRES occupancy");
 	CudaCheck(cudaStreamSynchronize(stream), "resident GMRES plan");
 	fits_ = resident >= 1 && ctas_ <= sms;
@@ -876,12 +975,21 @@ ResidentStatus ResidentKrylov::Solve(const ResidentProblem& problem, cudaStream_
 	args.pieces = pieces_;
 	args.ctas = ctas_;
 	args.groups = groups_;
+	args.keep = keep_;
 	args.max_cycles_iterations = kIterationsPerLaunch;
 	args.cta_row = cta_row_.get();
 	args.cta_group = cta_group_.get();
 	args.group_cta = group_cta_.get();
 	args.agg_list = agg_list_.get();
 	args.agg_list_offsets = agg_list_offsets_.get();
+	args.cta_parts = tables_[0].get();
+	args.part_start = tables_[1].get();
+	args.part_nodes = tables_[2].get();
+	args.part_offsets = tables_[3].get();
+	args.part_list = tables_[4].get();
+	args.group_agg = tables_[5].get();
+	args.group_agg_offsets = tables_[6].get();
+	args.coarse_part = coarse_part_.get();
 	args.partial = partial_.get();
 	args.R = R_.get();
 	args.y = y_.get();
@@ -894,7 +1002,7 @@ ResidentStatus ResidentKrylov::Solve(const ResidentProblem& problem, cudaStream_
 	for (;;) {
 		status_.Zero(stream);
 		void* parameters[] = {&args};
-		CudaCheck(cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(KernelOf(kind_)), dim3(ctas_), dim3(kThreads),
+		CudaCheck(cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(KernelOf(kind_)), dim3(ctas_), dim3(threads_),
 			parameters, smem_, stream), "ResidentKrylovKernel");
 		if (launches) *launches += 1;
 		CudaCheck(cudaMemcpyAsync(host_, args.status, sizeof(ResidentStatus), cudaMemcpyDeviceToHost, stream),

@@ -13,12 +13,9 @@ namespace tfiga {
 struct AmgResidentView {
 	int coarse = 0;                          // aggregates; 0: no AMG
 	const int32_t* agg = nullptr;            // aggregate of every fine node
-	const int32_t* agg_order = nullptr;      // fine nodes by aggregate, offsets agg_offsets
-	const int32_t* agg_offsets = nullptr;
 	const double* mask = nullptr;            // [4 nodes] 1 = free
 	const double* dense = nullptr;           // inverse of the coarse operator, rows dense_ld apart
 	long long dense_ld = 0;
-	double* coarse_rhs = nullptr;            // [4 coarse] scratch
 	double* coarse_x = nullptr;              // [4 coarse] scratch
 	const int32_t* ap_rows = nullptr;        // A P: block rows of the fine nodes
 	const int32_t* ap_cols = nullptr;
@@ -77,10 +74,13 @@ private:
 	Kind kind_ = kLeft4;
 	std::vector<int64_t> segments_;
 	long long amg_version_ = -1;
-	int ctas_ = 0, groups_ = 1, restart_ = 0, slice_ = 0, pieces_ = 1;
+	int ctas_ = 0, groups_ = 1, restart_ = 0, slice_ = 0, pieces_ = 1, threads_ = 0;
+	bool keep_ = false;
 	size_t smem_ = 0;
 	DeviceArray<int32_t> cta_row_, cta_group_, group_cta_, agg_list_, agg_list_offsets_;
-	DeviceArray<double> partial_, R_, y_, tolerance_;
+	static constexpr int kTables = 7;
+	DeviceArray<int32_t> tables_[kTables];   // restriction by CTA and group (see Args)
+	DeviceArray<double> partial_, R_, y_, tolerance_, coarse_part_;
 	DeviceArray<int> flags_;                 // group stop flags
 	DeviceArray<int32_t> status_;            // a ResidentStatus
 	ResidentStatus* host_ = nullptr;
