@@ -1,80 +1,93 @@
-// One 4x4 block row of A x, shared by the SpMV kernels and the AMG residual.
+// One 4x4 block row of A x.
 //
-// A warp owns one block row; lane l multiplies whole blocks l, l+32, ...
-// (16 FP32 values in four 128-bit loads, or 16 FP64 values in eight), so a
-// warp keeps 32 blocks of values in flight, and the column index of a lane's
-// next block is loaded one step ahead so that the x gather does not wait on
-// it.  The four row sums are then reduced across the warp (three butterfly
-// levels on all four, two reduce-scatter levels) so that lane r ends with row
-// r.  This replaces the reference's thread-per-row BlockSpmvKernel
-// (solvers/cuda/include/SparseKernels.cuh:25-40), whose loads are strided.
+// Four lanes share a block, one row of it each, so that a warp reads eight consecutive blocks at once, contiguously
+// (16 bytes per lane of FP32 values, two times 16 of FP64), and a row's sum needs three shuffles.  Several such
+// groups are in flight per warp.  With a whole block per lane the 16-byte loads of a warp lay 64 or 128 bytes apart:
+// FP64 products ran at 3.6 TB/s (2.4 GB matrix of 58,145 rows: 383 us, now 224), FP32 ones of matrices near the L2's
+// size at 4.8 TB/s (207 MB: 43 us, now 39).  kParts warps share a row where a warp per row would leave the chip's
+// schedulers idle; kStream: values are loaded to leave the L2 first (a matrix that does not fit it).
 #pragma once
 
 #include "kernels.cuh"
 
 namespace tfiga {
 
-template <class T> struct BlockLoad;
-template <> struct BlockLoad<double> {
-	static __device__ __forceinline__ void Get(const double* values, long long b, double a[16])
+template <bool kStream, class V> __device__ __forceinline__ V LoadMatrix(const V* p)
+{
+	if constexpr (kStream) return __ldcs(p);
+	else return __ldg(p);
+}
+
+// Row r of a 4x4 block, and its product with the block column's four vector entries added to s.
+template <class T> struct BlockRow;
+template <> struct BlockRow<float> {
+	float4 q;
+	template <bool kStream> __device__ __forceinline__ void Load(const float* v, size_t block, int r)
 	{
-		const double2* p = reinterpret_cast<const double2*>(values+(size_t)b*16);
-		#pragma unroll
-		for (int k = 0; k < 8; ++k) { const double2 v = __ldg(p+k); a[2*k] = v.x; a[2*k+1] = v.y; }
+		q = LoadMatrix<kStream>(reinterpret_cast<const float4*>(v+block*16+4*r));
+	}
+	__device__ __forceinline__ double Dot(double2 x, double2 y, double s) const
+	{
+		s = fma((double)q.x, x.x, s); s = fma((double)q.y, x.y, s);
+		return fma((double)q.w, y.y, fma((double)q.z, y.x, s));
 	}
 };
-template <> struct BlockLoad<float> {
-	static __device__ __forceinline__ void Get(const float* values, long long b, double a[16])
+template <> struct BlockRow<double> {
+	double2 a, b;
+	template <bool kStream> __device__ __forceinline__ void Load(const double* v, size_t block, int r)
 	{
-		const float4* p = reinterpret_cast<const float4*>(values+(size_t)b*16);
-		#pragma unroll
-		for (int k = 0; k < 4; ++k) {
-			const float4 v = __ldg(p+k);
-			a[4*k] = v.x; a[4*k+1] = v.y; a[4*k+2] = v.z; a[4*k+3] = v.w;
-		}
+		const double2* q = reinterpret_cast<const double2*>(v+block*16+4*r);
+		a = LoadMatrix<kStream>(q);
+		b = LoadMatrix<kStream>(q+1);
+	}
+	__device__ __forceinline__ double Dot(double2 x, double2 y, double s) const
+	{
+		s = fma(a.x, x.x, s); s = fma(a.y, x.y, s);
+		return fma(b.y, y.y, fma(b.x, y.x, s));
 	}
 };
 
-// Returns (A x)[4*row + r] in lane r = 0..3 of the warp (lane l holds row l & 3).
-template <class T>
-__device__ __forceinline__ double RowBlockDot(const DevicePatternView& p, const T* __restrict__ values,
-	const double* __restrict__ x, int row, int lane)
+// The sum of row r = lane & 3 over the warp's eight block groups.
+__device__ __forceinline__ double QuadRowSum(double s)
 {
-	double s0 = 0.0, s1 = 0.0, s2 = 0.0, s3 = 0.0;
-	const int hi = p.row_offsets[row+1];
-	int b = p.row_offsets[row]+lane;
-	int col = b < hi ? p.columns[b] : 0;
-	while (b < hi) {
-		const int next = b+32;
-		const int next_col = next < hi ? p.columns[next] : 0;
-		double a[16];
-		BlockLoad<T>::Get(values, b, a);
-		const double2* xv = reinterpret_cast<const double2*>(x+4*(size_t)col);
-		const double2 x01 = __ldg(xv), x23 = __ldg(xv+1);
-		s0 = fma(a[0], x01.x, s0); s0 = fma(a[1], x01.y, s0); s0 = fma(a[2], x23.x, s0); s0 = fma(a[3], x23.y, s0);
-		s1 = fma(a[4], x01.x, s1); s1 = fma(a[5], x01.y, s1); s1 = fma(a[6], x23.x, s1); s1 = fma(a[7], x23.y, s1);
-		s2 = fma(a[8], x01.x, s2); s2 = fma(a[9], x01.y, s2); s2 = fma(a[10], x23.x, s2); s2 = fma(a[11], x23.y, s2);
-		s3 = fma(a[12], x01.x, s3); s3 = fma(a[13], x01.y, s3); s3 = fma(a[14], x23.x, s3); s3 = fma(a[15], x23.y, s3);
-		b = next;
-		col = next_col;
-	}
 	#pragma unroll
-	for (int o = 16; o >= 4; o >>= 1) {
-		s0 += __shfl_xor_sync(0xffffffffu, s0, o);
-		s1 += __shfl_xor_sync(0xffffffffu, s1, o);
-		s2 += __shfl_xor_sync(0xffffffffu, s2, o);
-		s3 += __shfl_xor_sync(0xffffffffu, s3, o);
+	for (int o = 16; o >= 4; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+	return s;
+}
+
+// Part `part` of kParts of (A x)[4*row + r], in lanes with lane & 3 == r.
+template <class T, int kParts, bool kStream>
+__device__ __forceinline__ double RowBlockDot(const DevicePatternView& p, const T* __restrict__ values,
+	const double* __restrict__ x, int row, int part, int lane)
+{
+	// groups of eight blocks in flight: as many as registers and a part's length allow
+	constexpr int kUnroll = sizeof(T) == 4 ? 4 : kParts == 4 ? 2 : kParts == 1 && kStream ? 8 : 4;
+	const int b0 = p.row_offsets[row], b1 = p.row_offsets[row+1];
+	const int per = (b1-b0+kParts-1)/kParts;
+	const int lo = min(b1, b0+part*per), hi = min(b1, lo+per);
+	const int r = lane & 3;
+	double s = 0.0;
+	int b = lo+(lane >> 2);
+	for (; b+8*(kUnroll-1) < hi; b += 8*kUnroll) {
+		int c[kUnroll];
+		BlockRow<T> a[kUnroll];
+		#pragma unroll
+		for (int u = 0; u < kUnroll; ++u) c[u] = __ldg(p.columns+b+8*u);
+		#pragma unroll
+		for (int u = 0; u < kUnroll; ++u) a[u].template Load<kStream>(values, (size_t)(b+8*u), r);
+		#pragma unroll
+		for (int u = 0; u < kUnroll; ++u) {
+			const double2* v = reinterpret_cast<const double2*>(x+4*(size_t)c[u]);
+			s = a[u].Dot(__ldg(v), __ldg(v+1), s);
+		}
 	}
-	const bool upper = (lane & 2) != 0;            // keeps rows 2, 3
-	double k0 = upper ? s2 : s0, k1 = upper ? s3 : s1;
-	const double g0 = upper ? s0 : s2, g1 = upper ? s1 : s3;
-	k0 += __shfl_xor_sync(0xffffffffu, g0, 2);
-	k1 += __shfl_xor_sync(0xffffffffu, g1, 2);
-	const bool odd = (lane & 1) != 0;              // keeps rows 1, 3
-	double keep = odd ? k1 : k0;
-	const double give = odd ? k0 : k1;
-	keep += __shfl_xor_sync(0xffffffffu, give, 1);
-	return keep;
+	for (; b < hi; b += 8) {
+		const double2* v = reinterpret_cast<const double2*>(x+4*(size_t)__ldg(p.columns+b));
+		BlockRow<T> a;
+		a.template Load<kStream>(values, (size_t)b, r);
+		s = a.Dot(__ldg(v), __ldg(v+1), s);
+	}
+	return QuadRowSum(s);
 }
 
 } // namespace tfiga

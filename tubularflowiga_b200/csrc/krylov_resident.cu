@@ -28,6 +28,8 @@
 // every CTA returns.
 #include "krylov_resident.hpp"
 
+#include "block_row.cuh"
+
 #include <algorithm>
 #include <cmath>
 #include <type_traits>
@@ -109,49 +111,8 @@ __device__ __forceinline__ double2 Load2(const double* p)
 	return v;
 }
 
-// 4x4 blocks: four lanes share a block, one row each (a warp reads eight consecutive blocks at once, contiguously), so
-// a row's sum needs three shuffles; 2x2 blocks: a lane takes a whole block.
-template <bool kStream, class V> __device__ __forceinline__ V LoadMatrix(const V* p)
-{
-	if constexpr (kStream) return __ldcs(p);
-	else return __ldg(p);
-}
-template <class T> struct BlockRow;
-template <> struct BlockRow<float> {
-	float4 q;
-	template <bool kStream> __device__ __forceinline__ void Load(const float* v, size_t block, int r)
-	{
-		q = LoadMatrix<kStream>(reinterpret_cast<const float4*>(v+block*16+4*r));
-	}
-	__device__ __forceinline__ double Dot(double2 x, double2 y, double s) const
-	{
-		s = fma((double)q.x, x.x, s); s = fma((double)q.y, x.y, s);
-		return fma((double)q.w, y.y, fma((double)q.z, y.x, s));
-	}
-};
-template <> struct BlockRow<double> {
-	double2 a, b;
-	template <bool kStream> __device__ __forceinline__ void Load(const double* v, size_t block, int r)
-	{
-		const double2* q = reinterpret_cast<const double2*>(v+block*16+4*r);
-		a = LoadMatrix<kStream>(q);
-		b = LoadMatrix<kStream>(q+1);
-	}
-	__device__ __forceinline__ double Dot(double2 x, double2 y, double s) const
-	{
-		s = fma(a.x, x.x, s); s = fma(a.y, x.y, s);
-		return fma(b.y, y.y, fma(b.x, y.x, s));
-	}
-};
-
-__device__ __forceinline__ double QuadRowSum(double s)     // the row sum r in lanes with lane & 3 == r
-{
-	#pragma unroll
-	for (int o = 16; o >= 4; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-	return s;
-}
-
-// One piece of a block row, blocks lo .. hi - 1: the row sum r in lane r < F.
+// One piece of a block row, blocks lo .. hi - 1 (4x4: block_row.cuh; 2x2: a lane takes a whole block): the row sum r in
+// lane r < F.
 template <int F, class T, bool kStream>
 __device__ __forceinline__ double PieceSum(const T* values, const int32_t* cols, const double* x, int lo, int hi,
 	int lane)

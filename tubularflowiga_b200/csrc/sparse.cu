@@ -2,7 +2,7 @@
 // apply), diagonal-block inverse, Dirichlet rows, boundary-face flows and
 // tractions, and deterministic two-stage reductions.
 //
-// SpMV layout: one warp per block row (block_row.cuh).
+// SpMV layout: one warp, or a few, per block row (block_row.cuh).
 #include "block_row.cuh"
 #include "common.hpp"
 #include "kernels.cuh"
@@ -12,38 +12,69 @@ namespace {
 
 constexpr int kReduceBlocks = 296;   // 2 CTAs per SM for the partial-sum stage
 
-template <class T>
-__global__ void __launch_bounds__(256) SpmvKernel(DevicePatternView p, const T* __restrict__ values,
-	const double* __restrict__ x, double* __restrict__ y)
-{
-	const int row = blockIdx.x*8+(threadIdx.x >> 5);
-	const int lane = threadIdx.x & 31;
-	if (row >= p.nodes) return;
-	const double sum = RowBlockDot(p, values, x, row, lane);
-	if (lane < 4) y[4*(size_t)row+lane] = sum;
-}
+constexpr int kSpmvWarps = 8;        // warps per CTA
 
-template <class T>
-__global__ void __launch_bounds__(256) SpmvBlockJacobiKernel(DevicePatternView p, const T* __restrict__ values,
+// y = [D^-1] (scale * A x): inverse, scale, stop and the segments (node_seg, seg_stop: rows of stopped segments keep
+// their old y) are optional.
+template <class T, int kParts, bool kStream>
+__global__ void __launch_bounds__(32*kSpmvWarps) SpmvKernel(DevicePatternView p, const T* __restrict__ values,
 	const double* __restrict__ inverse, const double* __restrict__ x, const double* __restrict__ scale,
-	double* __restrict__ y, const int* __restrict__ stop)
+	double* __restrict__ y, const int* __restrict__ stop, const int32_t* __restrict__ node_seg,
+	const int* __restrict__ seg_stop)
 {
 	if (stop != nullptr && *stop) return;
-	const int row = blockIdx.x*8+(threadIdx.x >> 5);
-	const int lane = threadIdx.x & 31;
-	if (row >= p.nodes) return;
-	double sum = RowBlockDot(p, values, x, row, lane);
+	constexpr int kRows = kSpmvWarps/kParts;
+	const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+	int row = blockIdx.x*kRows+warp/kParts;
+	const auto skipped = [&](int r) { return r >= p.nodes || (seg_stop != nullptr && seg_stop[node_seg[r]]); };
+	double sum = 0.0;
+	if (!skipped(row)) sum = RowBlockDot<T, kParts, kStream>(p, values, x, row, warp%kParts, lane);
+	if constexpr (kParts > 1) {
+		// the parts of a row, four lanes per row in the first warp
+		__shared__ double parts[kSpmvWarps][4];
+		if (lane < 4) parts[warp][lane] = sum;
+		__syncthreads();
+		if (warp > 0) return;
+		row = blockIdx.x*kRows+(lane >> 2);
+		sum = 0.0;
+		if (lane < 4*kRows)
+			#pragma unroll
+			for (int k = 0; k < kParts; ++k) sum += parts[(lane >> 2)*kParts+k][lane & 3];
+	}
 	if (scale != nullptr) sum *= *scale;
-	if (inverse == nullptr) {
-		if (lane < 4) y[4*(size_t)row+lane] = sum;
-		return;
+	if (inverse != nullptr) {
+		const int base = lane & ~3;
+		const double y0 = __shfl_sync(0xffffffffu, sum, base), y1 = __shfl_sync(0xffffffffu, sum, base+1);
+		const double y2 = __shfl_sync(0xffffffffu, sum, base+2), y3 = __shfl_sync(0xffffffffu, sum, base+3);
+		if (row < p.nodes) {
+			const double* d = inverse+(size_t)row*16+(lane & 3)*4;
+			sum = d[0]*y0+d[1]*y1+d[2]*y2+d[3]*y3;
+		}
 	}
-	const double y0 = __shfl_sync(0xffffffffu, sum, 0), y1 = __shfl_sync(0xffffffffu, sum, 1);
-	const double y2 = __shfl_sync(0xffffffffu, sum, 2), y3 = __shfl_sync(0xffffffffu, sum, 3);
-	if (lane < 4) {
-		const double* d = inverse+(size_t)row*16+lane*4;
-		y[4*(size_t)row+lane] = d[0]*y0+d[1]*y1+d[2]*y2+d[3]*y3;
-	}
+	if (lane < (kParts > 1 ? 4*kRows : 4) && !skipped(row)) y[4*(size_t)row+(lane & 3)] = sum;
+}
+
+// A matrix of more than this many bytes is streamed past the L2 (126 MB).
+constexpr size_t kSpmvStreamBytes = (size_t)96 << 20;
+// Warps that fill the chip (64 on each of 148 SMs): rows are split while their parts do not exceed them (cylinder of
+// 1,681 rows, FP64: 14.4 us with a warp per row, 6.2 with four; 14,645 rows: 39 us with one, 41 with two).
+constexpr int kSpmvFill = 64*148;
+
+template <class T>
+void SpmvLaunch(const DevicePatternView& p, const T* values, const double* inverse, const double* x,
+	const double* scale, double* y, const int* stop, const int32_t* node_seg, const int* seg_stop, cudaStream_t stream)
+{
+	if (p.nodes == 0) return;
+	const auto launch = [&](auto kernel, int parts) {
+		const int rows = kSpmvWarps/parts;
+		kernel<<<(unsigned)((p.nodes+rows-1)/rows), 32*kSpmvWarps, 0, stream>>>(p, values, inverse, x, scale, y, stop,
+			node_seg, seg_stop);
+	};
+	if (4LL*p.nodes <= kSpmvFill) launch(SpmvKernel<T, 4, false>, 4);
+	else if (2LL*p.nodes <= kSpmvFill) launch(SpmvKernel<T, 2, false>, 2);
+	else if ((size_t)p.blocks*16*sizeof(T) <= kSpmvStreamBytes) launch(SpmvKernel<T, 1, false>, 1);
+	else launch(SpmvKernel<T, 1, true>, 1);
+	LaunchCheck("SpmvKernel");
 }
 
 // Gauss-Jordan with partial pivoting and the singular fallback of
@@ -286,42 +317,21 @@ int PartialSlots() { return 2*kReduceBlocks; }
 template <class T>
 void LaunchSpmv(const DevicePatternView& p, const T* values, const double* x, double* y, cudaStream_t stream)
 {
-	if (p.nodes == 0) return;
-	SpmvKernel<T><<<Blocks(p.nodes, 8), 256, 0, stream>>>(p, values, x, y);
-	LaunchCheck("SpmvKernel");
-}
-
-// y = A x on the block rows of segments still open (node_seg[row] the row's segment, seg_stop[s] set
-// once segment s has stopped: its rows are skipped and y there is left as it was).
-template <class T>
-__global__ void __launch_bounds__(256) SpmvMaskedKernel(DevicePatternView p, const T* __restrict__ values,
-	const double* __restrict__ x, double* __restrict__ y, const int* __restrict__ stop,
-	const int32_t* __restrict__ node_seg, const int* __restrict__ seg_stop)
-{
-	if (*stop) return;
-	const int row = blockIdx.x*8+(threadIdx.x >> 5);
-	const int lane = threadIdx.x & 31;
-	if (row >= p.nodes || seg_stop[node_seg[row]]) return;
-	const double sum = RowBlockDot(p, values, x, row, lane);
-	if (lane < 4) y[4*(size_t)row+lane] = sum;
+	SpmvLaunch<T>(p, values, nullptr, x, nullptr, y, nullptr, nullptr, nullptr, stream);
 }
 
 template <class T>
 void LaunchSpmvMasked(const DevicePatternView& p, const T* values, const double* x, double* y, const int* stop,
 	const int32_t* node_seg, const int* seg_stop, cudaStream_t stream)
 {
-	if (p.nodes == 0) return;
-	SpmvMaskedKernel<T><<<Blocks(p.nodes, 8), 256, 0, stream>>>(p, values, x, y, stop, node_seg, seg_stop);
-	LaunchCheck("SpmvMaskedKernel");
+	SpmvLaunch<T>(p, values, nullptr, x, nullptr, y, stop, node_seg, seg_stop, stream);
 }
 
 template <class T>
 void LaunchSpmvBlockJacobi(const DevicePatternView& p, const T* values, const double* inverse,
 	const double* x, const double* scale, double* y, const int* stop, cudaStream_t stream)
 {
-	if (p.nodes == 0) return;
-	SpmvBlockJacobiKernel<T><<<Blocks(p.nodes, 8), 256, 0, stream>>>(p, values, inverse, x, scale, y, stop);
-	LaunchCheck("SpmvBlockJacobiKernel");
+	SpmvLaunch<T>(p, values, inverse, x, scale, y, stop, nullptr, nullptr, stream);
 }
 
 template <class T>
