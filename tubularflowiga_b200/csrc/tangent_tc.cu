@@ -16,14 +16,17 @@
 // columns' different formulas), and a point's numbers are broadcast reads.  The two warps of a quarter take one of
 // a chunk's two depth steps each; both points of a pair run in the halves of the packed FP32 operations.
 // Chunks of eight points (two depth steps of K = 16: the waits and fences of a chunk cost a thread as much as a
-// quarter of its arithmetic on four points).  Eight warps build; a ninth has one thread that fetches the chunks (bulk copies,
-// three staged) and issues the MMAs.  They meet on mbarriers only (staged -> build -> full -> MMA -> empty; A and
+// quarter of its arithmetic on four points).  Eight warps build; a ninth has one thread that issues the MMAs, a tenth
+// (FP32 tables) one that fetches the chunks (bulk copies, three or four staged, across the items of a CTA: issuing them took the MMA thread
+// 1,000 cycles a chunk).  They meet on mbarriers only (staged -> build -> unstaged, and full -> MMA -> empty; A and
 // Psi, in shared memory with the 64-byte swizzle, are double-buffered): with a block barrier a chunk and one of the
 // builders issuing, every chunk waited for that warp (37,000 cycles per CTA of which 12,000 waiting).  Waits are
-// bounded by %globaltimer.  Two CTAs per SM (256 tensor-memory columns each).
+// bounded in clock cycles.  Two CTAs per SM (256 tensor-memory columns each).
 // Functions past the element's own are left out of N (steps of 16) and, from 32 down, of the second warp half.
-// Epilogue: 16 columns a at a time through shared memory, so that a thread has all four column fields of a block
-// and adds 16 bytes at once (red.global.add.v4.f32).
+// Epilogue: 16 columns a at a time through shared memory (a barrier a round where two rounds' worth fits), so that a thread has all
+// four column fields of a block and adds 16 bytes at once (red.global.add.v4.f32).  Adding 8 bytes straight from the
+// accumulators, without the barriers, is slower (tube below 6.09 ms against 5.80): the L2's additions per sector count.
+// Cycles of an item (64 functions, two CTAs on the SM): build 11,000, Psi 2,500, epilogue 7,000, waits 6,500.
 //
 // Operands: BF16, split BF16 (hi + lo, three products) or TF32.
 // Basis values come from the FP32 copy of the tables (coefficients / element organisation: one CTA per element and
@@ -31,8 +34,8 @@
 // needs no copy).
 //
 // Measured, split BF16, against the kernel this replaces (G from 320 coefficients per point, through shared memory):
-// 25,600-element tube 6.64 -> 5.80 ms, 3,264-element bifurcation 0.87 -> 0.72 ms; the coefficients it needed cost the
-// point kernel 2.41 ms (now 1.05 ms) and 80 KiB per element (now 18).  From the FP64 tables 8.7 ms (before: 2.5 times
+// 25,600-element tube 6.64 -> 5.57 ms, 3,264-element bifurcation 0.87 -> 0.69 ms; the coefficients it needed cost the
+// point kernel 2.41 ms (now 1.05 ms) and 80 KiB per element (now 18).  From the FP64 tables 8.0 ms (before: 2.5 times
 // the other organisation).
 #include "common.hpp"
 #include "kernels.cuh"
@@ -45,23 +48,27 @@ namespace tfiga {
 namespace {
 
 constexpr int kBuilders = 256;                   // building threads
-constexpr int kThreads = kBuilders+32;           // and the fetching and issuing warp
+// and a warp that issues the MMAs, and one that fetches; from the FP64 tables there is little to fetch (8.5 ms for the
+// tube above with the warp, 8.0 without)
+constexpr int Threads(bool fp64_tables) { return kBuilders+(fp64_tables ? 32 : 64); }
 constexpr int kPoints = 8;                       // points per chunk: two depth steps of K = 16
 constexpr int kChunks = kQuad/kPoints;
-constexpr int kSlots = 3;                        // staged chunks
 constexpr int kTmemCols = 256;                   // D: 2 x 64, A: 2 buffers x 2 depth steps x 2 tiles x 16
 constexpr int kTmemA = 128;
-constexpr unsigned long long kWaitNs = 1000000000ull;
+constexpr long long kWaitCycles = 2000000000;   // about a second
 constexpr int kEpilogueColumns = 16;
 
 constexpr int kModeBf16 = 0, kModeSplit = 1, kModeTf32 = 2;
 
-struct __align__(1024) TangentShared {
+// Staged chunks, and epilogue rounds in shared memory: from the FP64 tables, which go through the L1, a slot and a round
+// more cost more than they give (25,600-element tube 9.25 ms with four and two, 8.6 with three and one).
+template <bool kFp64Tables> struct __align__(1024) TangentShared {
+	static constexpr int kSlots = kFp64Tables ? 3 : 4, kRounds = kFp64Tables ? 1 : 2;
 	unsigned char psi[2][2][64*64];              // B operand of a depth step: 64 rows a x 64 bytes, swizzled
 	float2 phi[kSlots][kFeatures][kPoints/2][kMaxBasis];   // point pairs
 	float2 pack[kSlots][kPoints/2][kPack];
-	float out[4][kEpilogueColumns][kMaxBasis];   // [column field][a][b]
-	uint64_t staged[kSlots], full[2], empty[2];
+	float out[kRounds][4][kEpilogueColumns][kMaxBasis];   // rounds of [column field][a][b]
+	uint64_t staged[kSlots], unstaged[kSlots], full[2], empty[2];
 	uint32_t tmem;
 };
 constexpr uint32_t kPhiBytes = kPoints/2*kMaxBasis*8;      // one feature of a chunk
@@ -93,13 +100,6 @@ __device__ __forceinline__ int Sw64(int r, int j)
 	return r*64+((j ^ ((r >> 1) & 3)) << 4);
 }
 
-__device__ __forceinline__ unsigned long long GlobalTimer()
-{
-	unsigned long long t;
-	asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-	return t;
-}
-
 __device__ __forceinline__ void MbarInit(uint64_t* bar, uint32_t count)
 {
 	asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" :: "r"(SmemAddress(bar)), "r"(count) : "memory");
@@ -124,24 +124,27 @@ __device__ __forceinline__ void BulkCopy(void* dst, const void* src, uint32_t by
 		:: "r"(SmemAddress(dst)), "l"(src), "r"(bytes), "r"(SmemAddress(bar)) : "memory");
 }
 
-__device__ __forceinline__ bool MbarTryWait(uint64_t* bar, uint32_t parity)
+__device__ __forceinline__ bool MbarTryWait(uint32_t bar, uint32_t parity)
 {
 	uint32_t done;
 	asm volatile("{\n\t.reg .pred p;\n\t"
 		"mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
 		"selp.u32 %0, 1, 0, p;\n\t}"
-		: "=r"(done) : "r"(SmemAddress(bar)), "r"(parity) : "memory");
+		: "=r"(done) : "r"(bar), "r"(parity) : "memory");
 	return done != 0;
 }
 
-// Waits for completion of the mbarrier phase with the given parity, for at most kWaitNs.
-__device__ bool MbarWaitBounded(uint64_t* bar, uint32_t parity)
+// Waits for completion of the mbarrier phase with the given parity, for at most kWaitCycles.
+__device__ __noinline__ bool MbarWaitLonger(uint32_t bar, uint32_t parity)
 {
-	if (MbarTryWait(bar, parity)) return true;   // (reading the timer is slow)
-	const unsigned long long start = GlobalTimer();
+	const long long start = clock64();
 	while (!MbarTryWait(bar, parity))
-		if (GlobalTimer()-start > kWaitNs) return false;
+		if (clock64()-start > kWaitCycles) return false;
 	return true;
+}
+__device__ __forceinline__ bool MbarWaitBounded(uint64_t* bar, uint32_t parity)
+{
+	return MbarTryWait(SmemAddress(bar), parity) || MbarWaitLonger(SmemAddress(bar), parity);
 }
 
 // D (128 x N, FP32) (+)= A (128 x K, in tensor memory) B^T (N x K, in shared memory): K = 16 BF16 or 8 TF32.
@@ -291,8 +294,8 @@ struct PairReader {
 // Both of the thread's columns (fields kHalf and 2 + kHalf: tiles 0 and 1, sixteen columns apart) at the depth
 // step's two point pairs, into its row of A.  Columns of a depth step: BF16 pairs of the points' hi parts, pair by
 // pair and feature by feature, then the lo parts eight columns on; TF32: two columns per pair and feature.
-template <int kMode, int I, int kHalf>
-__device__ __forceinline__ void BuildRows(const TangentShared& sm, int slot, int step, int b, Pair irho, Pair minus_nu,
+template <int kMode, int I, int kHalf, class Shared>
+__device__ __forceinline__ void BuildRows(const Shared& sm, int slot, int step, int b, Pair irho, Pair minus_nu,
 	uint32_t column)
 {
 	uint32_t r[2][16];
@@ -331,23 +334,30 @@ __device__ __forceinline__ void BuildRows(const TangentShared& sm, int slot, int
 }
 
 template <int kMode, bool kFp64Tables>
-__global__ void __launch_bounds__(kThreads, 2) TangentKernel(DeviceMeshView mesh, int items,
+__global__ void __launch_bounds__(Threads(kFp64Tables), 2) TangentKernel(DeviceMeshView mesh, int items,
 	const float* __restrict__ phi32, const double* __restrict__ phi64, const float* __restrict__ packs,
 	const int32_t* __restrict__ element_blocks, float irho_value, float minus_nu_value, float* __restrict__ values,
 	int* __restrict__ status)
 {
 	extern __shared__ unsigned char raw[];
-	TangentShared& sm = *reinterpret_cast<TangentShared*>(
+	using Shared = TangentShared<kFp64Tables>;
+	constexpr int kFetcher = kFp64Tables ? kBuilders : kBuilders+32;   // thread
+	constexpr int kSlots = Shared::kSlots, kRounds = Shared::kRounds;
+	Shared& sm = *reinterpret_cast<Shared*>(
 		(reinterpret_cast<uintptr_t>(raw)+1023) & ~static_cast<uintptr_t>(1023));
 	const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
 	const int quarter = warp & 3, group = warp >> 2;     // a quarter's two warps: depth steps, then tiles
+	const auto functions = [&](int item) { return mesh.element_offsets[(item >> 2)+1]-mesh.element_offsets[item >> 2]; };
 	if (warp == 0) {
 		asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
 			:: "r"(SmemAddress(&sm.tmem)), "r"((uint32_t)kTmemCols) : "memory");
 		asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
 	}
 	if (tid == 0) {
-		for (int k = 0; k < kSlots; ++k) MbarInit(&sm.staged[k], 1);
+		for (int k = 0; k < kSlots; ++k) {
+			MbarInit(&sm.staged[k], 1);
+			MbarInit(&sm.unstaged[k], kBuilders/32);
+		}
 		for (int k = 0; k < 2; ++k) {
 			MbarInit(&sm.full[k], kBuilders/32);
 			MbarInit(&sm.empty[k], 1);
@@ -360,33 +370,50 @@ __global__ void __launch_bounds__(kThreads, 2) TangentKernel(DeviceMeshView mesh
 	const Pair irho{Pack2(irho_value, irho_value)}, minus_nu{Pack2(minus_nu_value, minus_nu_value)};
 	const int b = 32*(quarter & 1)+lane;
 	bool failed = false;
+	int ahead_nen = kFp64Tables ? 0 : functions(blockIdx.x);   // the next item's
 	int first = 0;                               // chunks of the items before this one
+
+	// Chunk number n of this CTA (counted over its items): slot n % kSlots, use n / kSlots of it; buffer n & 1, use
+	// n / 2.  Chunks are fetched in this order across the items, so that an item's first ones arrive during the
+	// epilogue before it.
+	int fetched = 0;
+	auto fetch = [&]() {
+		const long long item = blockIdx.x+(long long)(fetched/kChunks)*gridDim.x;
+		if (item >= items) return false;
+		const int e = (int)(item >> 2), c = fetched%kChunks, slot = fetched%kSlots;
+		MbarExpect(&sm.staged[slot], (kFp64Tables ? 0u : kFeatures*kPhiBytes)+kPackBytes);
+		if constexpr (!kFp64Tables) {
+			const float* P32 = phi32+(size_t)e*kFeatures*kQuad*kMaxBasis;
+			#pragma unroll
+			for (int t = 0; t < kFeatures; ++t)
+				BulkCopy(&sm.phi[slot][t][0][0], P32+((size_t)t*(kQuad/2)+c*(kPoints/2))*kMaxBasis*2, kPhiBytes,
+					&sm.staged[slot]);
+		}
+		BulkCopy(&sm.pack[slot][0][0], packs+(size_t)e*kQuad*kPack+(size_t)c*kPoints*kPack, kPackBytes, &sm.staged[slot]);
+		++fetched;
+		return true;
+	};
+
+	if constexpr (kFp64Tables)
+		if (tid == kFetcher)
+			for (int c = 0; c < kSlots; ++c) fetch();
 
 	for (int item = blockIdx.x; item < items; item += gridDim.x, first += kChunks) {
 		const int e = item >> 2, row = item & 3;
-		const int nen = mesh.element_offsets[e+1]-mesh.element_offsets[e];
+		int nen;
+		if constexpr (kFp64Tables) {             // (no registers to spare)
+			nen = functions(item);
+		} else {
+			nen = ahead_nen;
+			if ((long long)item+gridDim.x < items) ahead_nen = functions(item+gridDim.x);
+		}
 		const int columns = (nen+15) & ~15;      // N of the product
-		// chunk number n of this CTA (counted over its items): slot n % 3, use n / 3 of it; buffer n & 1, use n / 2
 		const auto wait = [&](uint64_t* bar, int use) {
 			if (!failed) failed = !MbarWaitBounded(bar, (uint32_t)(use & 1));
 		};
 		if (warp == kBuilders/32) {
 			if (lane == 0) {
-				const float* P32 = kFp64Tables ? nullptr : phi32+(size_t)e*kFeatures*kQuad*kMaxBasis;
-				const float* PK = packs+(size_t)e*kQuad*kPack;
 				const uint32_t idesc = InstructionDescriptor(kMode == kModeTf32, columns);
-				auto stage = [&](int c) {
-					const int slot = (first+c)%kSlots;
-					MbarExpect(&sm.staged[slot], (kFp64Tables ? 0u : kFeatures*kPhiBytes)+kPackBytes);
-					if constexpr (!kFp64Tables) {
-						#pragma unroll
-						for (int t = 0; t < kFeatures; ++t)
-							BulkCopy(&sm.phi[slot][t][0][0], P32+((size_t)t*(kQuad/2)+c*(kPoints/2))*kMaxBasis*2, kPhiBytes,
-								&sm.staged[slot]);
-					}
-					BulkCopy(&sm.pack[slot][0][0], PK+(size_t)c*kPoints*kPack, kPackBytes, &sm.staged[slot]);
-				};
-				for (int c = 0; c < kSlots; ++c) stage(c);
 				for (int c = 0; c < kChunks; ++c) {
 					const int buffer = c & 1;
 					wait(&sm.full[buffer], (first+c) >> 1);
@@ -396,26 +423,34 @@ __global__ void __launch_bounds__(kThreads, 2) TangentKernel(DeviceMeshView mesh
 						const uint64_t psi = DescSw64(SmemAddress(sm.psi[buffer][step]));
 						const uint64_t psi_next = DescSw64(SmemAddress(sm.psi[buffer][step])+32);
 						const uint32_t accumulate = c > 0 || step > 0 ? 1u : 0u;
-						#pragma unroll
-						for (int tile = 0; tile < 2; ++tile) {
-							const uint32_t d = tmem+64*tile, a = tmem+kTmemA+64*buffer+32*step+16*tile;
-							if constexpr (kMode == kModeTf32) {
-								MmaTf32(d, a, psi, idesc, accumulate);
-								MmaTf32(d, a+8, psi_next, idesc, 1u);
-							} else {
-								MmaBf16(d, a, psi, idesc, accumulate);                // hi hi
-								if constexpr (kMode == kModeSplit) {
-									MmaBf16(d, a, psi_next, idesc, 1u);               // hi lo
-									MmaBf16(d, a+8, psi, idesc, 1u);                  // lo hi
-								}
-							}
+						const uint32_t a = tmem+kTmemA+64*buffer+32*step;
+						// the tiles in turn: consecutive products accumulate into different columns
+						const auto both = [&](uint32_t offset, uint64_t operand, uint32_t add) {
+							#pragma unroll
+							for (int tile = 0; tile < 2; ++tile)
+								if constexpr (kMode == kModeTf32) MmaTf32(tmem+64*tile, a+16*tile+offset, operand, idesc, add);
+								else MmaBf16(tmem+64*tile, a+16*tile+offset, operand, idesc, add);
+						};
+						both(0, psi, accumulate);                              // hi hi; TF32: the first eight k
+						if constexpr (kMode == kModeSplit) {
+							both(0, psi_next, 1u);                             // hi lo
+							both(8, psi, 1u);                                  // lo hi
 						}
+						if constexpr (kMode == kModeTf32) both(8, psi_next, 1u);
 					}
 					MmaCommit(&sm.empty[buffer]);
 					// every builder is done with chunk c's slot
-					if (c+kSlots < kChunks) stage(c+kSlots);
+					if constexpr (kFp64Tables) if (!failed) fetch();
 				}
 			}
+			__syncwarp();
+		} else if (warp > kBuilders/32) {
+			// up to kSlots chunks ahead of the builders, into the next item
+			if (lane == 0)
+				while (fetched < first+kChunks+kSlots && !failed) {
+					if (fetched >= kSlots) wait(&sm.unstaged[fetched%kSlots], fetched/kSlots-1);
+					if (failed || !fetch()) break;
+				}
 			__syncwarp();
 		} else {
 		const double* P64 = kFp64Tables ? phi64+(size_t)e*kFeatures*kQuad*kMaxBasis : nullptr;
@@ -498,12 +533,11 @@ __global__ void __launch_bounds__(kThreads, 2) TangentKernel(DeviceMeshView mesh
 			FenceBeforeSync();
 			FenceProxyAsync();
 			__syncwarp();
-			if (lane == 0) MbarArrive(&sm.full[buffer]);
+			if (lane == 0) {
+				MbarArrive(&sm.full[buffer]);
+				if constexpr (!kFp64Tables) MbarArrive(&sm.unstaged[slot]);
+			}
 		}
-		// the last commits of both buffers, before the accumulators are read
-		wait(&sm.empty[0], ((first+kChunks) >> 1)-1);
-		wait(&sm.empty[1], ((first+kChunks) >> 1)-1);
-		FenceAfterSync();
 
 		// warp (tile, quarter): column field 2 tile + (quarter >> 1) of functions b for sixteen a at a time
 		const int field = 2*group+(quarter >> 1);
@@ -519,12 +553,17 @@ __global__ void __launch_bounds__(kThreads, 2) TangentKernel(DeviceMeshView mesh
 		};
 		int block[4];
 		blocks_of(0, block);
+		// the last commits of both buffers, before the accumulators are read
+		wait(&sm.empty[0], ((first+kChunks) >> 1)-1);
+		wait(&sm.empty[1], ((first+kChunks) >> 1)-1);
+		FenceAfterSync();
 		for (int a0 = 0; a0 < columns; a0 += kEpilogueColumns) {
+			const int round = a0/kEpilogueColumns%kRounds;   // (two: its last readers have passed a barrier since)
 			if (32*(quarter & 1) < nen) {
 				float v[16];
 				TmemLoad16(tmem+((uint32_t)(32*quarter) << 16)+64*group+a0, v);
 				#pragma unroll
-				for (int k = 0; k < 16; ++k) sm.out[field][k][b] = v[k];
+				for (int k = 0; k < 16; ++k) sm.out[round][field][k][b] = v[k];
 			}
 			int ahead[4] = {-1, -1, -1, -1};
 			if (a0+kEpilogueColumns < columns) blocks_of(a0+kEpilogueColumns, ahead);
@@ -532,9 +571,9 @@ __global__ void __launch_bounds__(kThreads, 2) TangentKernel(DeviceMeshView mesh
 			#pragma unroll
 			for (int k = 0; k < 4; ++k)
 				if (block[k] >= 0)
-					RedAdd4(base+(size_t)block[k]*16, sm.out[0][oa+4*k][ob], sm.out[1][oa+4*k][ob], sm.out[2][oa+4*k][ob],
-						sm.out[3][oa+4*k][ob]);
-			builders_sync();
+					RedAdd4(base+(size_t)block[k]*16, sm.out[round][0][oa+4*k][ob], sm.out[round][1][oa+4*k][ob],
+						sm.out[round][2][oa+4*k][ob], sm.out[round][3][oa+4*k][ob]);
+			if constexpr (kRounds == 1) builders_sync();
 			#pragma unroll
 			for (int k = 0; k < 4; ++k) block[k] = ahead[k];
 		}
@@ -544,6 +583,8 @@ __global__ void __launch_bounds__(kThreads, 2) TangentKernel(DeviceMeshView mesh
 		if (__syncthreads_or(failed)) { failed = true; break; }
 		FenceAfterSync();
 	}
+	if (failed && tid == kFetcher)               // copies in flight land before the CTA ends
+		for (int n = max(0, fetched-kSlots); n < fetched; ++n) MbarWaitBounded(&sm.staged[n%kSlots], n/kSlots & 1);
 	__syncthreads();
 	if (failed && tid == 0) atomicOr(status, 1);
 	if (warp == 0)
@@ -558,7 +599,7 @@ void Launch(const DeviceMeshView& mesh, const float* phi32, const double* phi64,
 	const long long items = 4LL*mesh.elements;
 	if (items == 0) return;
 	if (items > 0x7fffffffLL) Fail(-7, "too many elements for one tangent launch");
-	const int bytes = (int)sizeof(TangentShared)+1024;
+	const int bytes = (int)sizeof(TangentShared<kFp64Tables>)+1024;
 	CudaCheck(cudaFuncSetAttribute(TangentKernel<kMode, kFp64Tables>, cudaFuncAttributeMaxDynamicSharedMemorySize,
 		bytes), "tangent shared memory");
 	long long grid = items;
@@ -568,7 +609,7 @@ void Launch(const DeviceMeshView& mesh, const float* phi32, const double* phi64,
 		CudaCheck(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device), "device attribute");
 		grid = std::min<long long>(items, 2LL*sms);
 	}
-	TangentKernel<kMode, kFp64Tables><<<(unsigned)grid, kThreads, bytes, stream>>>(mesh, (int)items, phi32, phi64,
+	TangentKernel<kMode, kFp64Tables><<<(unsigned)grid, Threads(kFp64Tables), bytes, stream>>>(mesh, (int)items, phi32, phi64,
 		packs, element_blocks, (float)(1.0/params.density), (float)(-params.viscosity/params.density), values, status);
 	LaunchCheck("TangentKernel");
 }
