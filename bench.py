@@ -1145,10 +1145,10 @@ def main():
                              "avg_ms": asm_ms / asm_n, "share": asm_ms / prof_ms,
                              "peak_note": "nominal B200 FP64 (no measured FP64 peak on this pool)"}
     if res_n:
-        # FP64 residual (+ point coefficients in the tensor-core modes): per element it reads the FP64
+        # FP64 residual (+ the tangent's numbers in the tensor-core modes): per element it reads the FP64
         # basis tables (5 x 64 x 64 doubles) and the point data (64 x 11 doubles) and, in the tensor-core
-        # modes, writes the coefficients of four row fields (4 x 80 x 64 floats)
-        rbytes = tube.mesh.elements * (5 * 64 * 64 * 8 + 64 * 11 * 8 + (4 * 80 * 64 * 4 if mixed else 0))
+        # modes, writes 72 numbers per point (72 x 64 floats)
+        rbytes = tube.mesh.elements * (5 * 64 * 64 * 8 + 64 * 11 * 8 + (72 * 64 * 4 if mixed else 0))
         a = rbytes / (res_ms / res_n * 1e-3) / 1e9
         kernels["residual_point"] = {"bound": "hbm", "achieved": a, "peak": hbm, "unit": "GB/s", "frac": a / hbm,
                                      "traffic": None, "launches": res_n, "avg_ms": res_ms / res_n,

@@ -166,11 +166,6 @@ __device__ __forceinline__ double PieceSum(const T* values, const int32_t* cols,
 	}
 }
 
-template <class B> __device__ __forceinline__ double BasisLoad(const B* p)
-{
-	return (double)*reinterpret_cast<const volatile B*>(p);
-}
-
 // Doubles that the own rows' offsets take (even, so that what follows stays 16-byte aligned).
 __host__ __device__ constexpr int RowSlots(int slice, int fields) { return ((slice/fields+2)/2+2) & ~1; }
 
@@ -765,7 +760,11 @@ bool ResidentKrylov::Prepare(Kind kind, const DevicePatternView& pattern, int re
 	amg_version_ = version;
 	segments_ = segments;
 	fits_ = false;
-	Plan(pattern, amg, stream);
+	try {
+		Plan(pattern, amg, stream);
+	} catch (const Error& error) {
+		if (error.status != -8) throw;       // no memory for the work arrays: the separate launches need none of them
+	}
 	planned_ = true;
 	return fits_;
 }

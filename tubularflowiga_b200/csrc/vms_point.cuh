@@ -1,5 +1,5 @@
-// Per-quadrature-point VMS Navier-Stokes quantities shared by the FP64
-// assembly kernel and the tensor-core tangent kernel.
+// Per-quadrature-point VMS Navier-Stokes quantities as coefficients of the products of basis values, for the
+// elements with more than 64 basis functions (the others take the factored form, vms_tangent.cuh).
 //
 // Formulation: the reference's BuildNavierStokesElementFromPreparedPoints
 // (solvers/cpu/include/NavierStokesElement.hpp:149-317, LegacyBodyFitted weak
@@ -25,15 +25,10 @@ struct PointState {
 };
 
 // Coefficients of row field i at one point, all scaled by the point
-// measure: M[((f - f_lo)*20 + s*5 + t)*kStride] multiplies (test feature s
-// of N_a) x (trial feature t of N_b) in K^{if}_{ab}; rc[s] = -measure * c_s
-// gives the residual.  Computed in FP64; C is the storage type of M (double
-// for the FP64 tangent, float for the tensor-core tangent).  Only the column
-// fields f in [f_lo, f_hi) are written; rc may be null.  kTangent false: only
-// rc is computed (M is not touched and may be null).
-template <class C, int kStride = 1, bool kTangent = true>
+// measure: M[f*20 + s*5 + t] multiplies (test feature s of N_a) x (trial
+// feature t of N_b) in K^{if}_{ab}; rc[s] = -measure * c_s gives the residual.
 __device__ __forceinline__ void RowCoefficients(int i, const PointState& S, const double* qd,
-	const AssemblyParams& prm, C* M, double* rc, int f_lo = 0, int f_hi = 4)
+	const AssemblyParams& prm, double* M, double* rc)
 {
 	const double rho = prm.density, mu = prm.viscosity, nu = mu/rho;
 	const double dt = prm.dt;
@@ -64,8 +59,7 @@ __device__ __forceinline__ void RowCoefficients(int i, const PointState& S, cons
 	const double divu = S.gv[0][0]+S.gv[1][1]+S.gv[2][2];
 	const double fine_p = -rho*tau_c*divu;
 	// Residual (:218-239).
-	if (rc == nullptr) {
-	} else if (i < 3) {
+	if (i < 3) {
 		double cN = rho*dudt[i];
 		for (int d = 0; d < 3; ++d) cN += rho*a[d]*S.gv[i][d];
 		rc[0] = -meas*cN;
@@ -78,7 +72,6 @@ __device__ __forceinline__ void RowCoefficients(int i, const PointState& S, cons
 		rc[0] = -meas*divu;
 		for (int d = 0; d < 3; ++d) rc[1+d] = meas*fine[d];
 	}
-	if constexpr (!kTangent) return;
 	// Exact tangent (:248-312), collected by (test, trial) feature.
 	const double t3 = tau_m*tau_m*tau_m;
 	double dtau_c[3], A[3][3];
@@ -88,12 +81,10 @@ __device__ __forceinline__ void RowCoefficients(int i, const PointState& S, cons
 		for (int c = 0; c < 3; ++c)
 			A[c][f] = -dtau_m*R[c]-tau_m*((c == f ? idt : 0.0)+S.gv[c][f]);
 	}
-	for (int k = 0; k < (f_hi-f_lo)*20; ++k) M[k*kStride] = C(0);
-	auto at = [&](int f, int s, int t) -> C& { return M[((f-f_lo)*20+s*5+t)*kStride]; };
-	const int f_vel = f_hi < 3 ? f_hi : 3;     // end of the velocity columns in range
-	const bool p_col = f_hi > 3;               // pressure column in range
+	for (int k = 0; k < kCoef; ++k) M[k] = 0.0;
+	auto at = [&](int f, int s, int t) -> double& { return M[f*20+s*5+t]; };
 	if (i < 3) {
-		for (int f = f_lo; f < f_vel; ++f) {
+		for (int f = 0; f < 3; ++f) {
 			double nn = rho*S.gv[i][f]+(f == i ? rho*idt : 0.0);
 			for (int d = 0; d < 3; ++d) nn += rho*A[d][f]*S.gv[i][d];
 			at(f, 0, 0) = nn;
@@ -114,24 +105,21 @@ __device__ __forceinline__ void RowCoefficients(int i, const PointState& S, cons
 				at(f, 1+d, 4) = -rho*tau_m*nu*((f == i ? a[d] : 0.0)+(d == f ? fine[i] : 0.0));
 			}
 		}
-		if (p_col) {
-			at(3, 1+i, 0) = -1.0;
-			for (int e = 0; e < 3; ++e) at(3, 0, 1+e) = -tau_m*S.gv[i][e];
-			for (int d = 0; d < 3; ++d)
-				for (int e = 0; e < 3; ++e)
-					at(3, 1+d, 1+e) = tau_m*((e == i ? a[d] : 0.0)+(d == e ? fine[i] : 0.0));
-		}
+		at(3, 1+i, 0) = -1.0;
+		for (int e = 0; e < 3; ++e) at(3, 0, 1+e) = -tau_m*S.gv[i][e];
+		for (int d = 0; d < 3; ++d)
+			for (int e = 0; e < 3; ++e)
+				at(3, 1+d, 1+e) = tau_m*((e == i ? a[d] : 0.0)+(d == e ? fine[i] : 0.0));
 	} else {
-		for (int f = f_lo; f < f_vel; ++f) {
+		for (int f = 0; f < 3; ++f) {
 			at(f, 0, 1+f) = 1.0;
 			for (int d = 0; d < 3; ++d) at(f, 1+d, 0) = -A[d][f];
 			for (int e = 0; e < 3; ++e) at(f, 1+f, 1+e) = tau_m*S.u[e];
 			at(f, 1+f, 4) = -tau_m*nu;
 		}
-		if (p_col)
-			for (int d = 0; d < 3; ++d) at(3, 1+d, 1+d) = tau_m/rho;
+		for (int d = 0; d < 3; ++d) at(3, 1+d, 1+d) = tau_m/rho;
 	}
-	for (int k = 0; k < (f_hi-f_lo)*20; ++k) M[k*kStride] = C(M[k*kStride]*meas);
+	for (int k = 0; k < kCoef; ++k) M[k] *= meas;
 }
 
 } // namespace tfiga
