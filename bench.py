@@ -639,7 +639,8 @@ def run_transport(args, world, rank, local):
             torch.cuda.synchronize()
         l1 = api.C.c_int64()
         api.check(lib.tfiga_transport_info(h, None, None, api.C.byref(l1)))
-        fam_ms, fam_n = np.zeros(5), np.zeros(5, np.int64)
+        families = len(api.NavierStokes.FAMILIES)      # what tfiga_transport_profile writes
+        fam_ms, fam_n = np.zeros(families), np.zeros(families, np.int64)
         if profile:
             api.check(lib.tfiga_transport_profile(h, api.C.c_void_p(fam_ms.ctypes.data),
                                                   api.C.c_void_p(fam_n.ctypes.data), 1))
