@@ -205,6 +205,15 @@ def replica_throughput(world, steps, ms):
     return world * steps / (ms / 1e3)
 
 
+def profile_pass(ms_per_step, launches, timed_launches):
+    """What the kernel figures were taken from: a repeat of the timed steps with events between the kernels."""
+    return {"ms_per_step": ms_per_step, "gpu_launches": launches, "timed_gpu_launches": timed_launches,
+            "note": "kernel families timed in a repeat of the timed steps; shares are of that pass's duration.  "
+                    "Profiled linear solves run as separate launches: where the timed steps solve in one launch "
+                    "(systems whose Krylov basis fits shared memory; fewer launches there), the Krylov, SpMV and "
+                    "AMG families are those of the separate kernels, not of the timed ones"}
+
+
 def step_dt(name):
     """Time step of a workload: the 1,280-element cylinder 1e-3 s; the tube batch 1e-4 s, because its
     smallest fast tubes (R 0.5 mm at Re 800, about 1.5 m/s) reach an axial CFL of 70 at 2e-3 s;
@@ -651,7 +660,8 @@ def run_transport(args, world, rank, local):
                 "fam_ms": fam_ms, "fam_n": fam_n, "clocks": clocks.summary(), "state": state,
                 "assembly_ms": assembly_ms.value}
 
-    run = timed(params, profile=True)
+    # the headline run is a caller's: no instrumentation (a profiled handle never takes the one-launch solve)
+    run = timed(params, profile=False)
     left = previous = None
     if not args.no_cpu_baseline and world == 1 and rank == 0:
         left = np.zeros(4 * mesh.blocks)
@@ -659,6 +669,9 @@ def run_transport(args, world, rank, local):
         api.check(lib.tfiga_transport_matrices(run["h"], api.C.c_void_p(left.ctypes.data),
                                                api.C.c_void_p(previous.ctypes.data)))
     api.check(lib.tfiga_transport_destroy(run["h"]))
+    # the same steps on a fresh handle with per-family events, for the kernel figures
+    prof = timed(params, profile=True)
+    api.check(lib.tfiga_transport_destroy(prof["h"]))
     fp64_leg = None
     if fp32 and not args.no_fp64_leg:
         ref = timed(make_params(api.FP64), profile=False)
@@ -687,8 +700,8 @@ def run_transport(args, world, rank, local):
     hbm, _, peak_kind = peaks()
     timed_report = run["report"]
     its_per_step = timed_report["total_iterations"] / max(args.steps, 1)
-    spmv_ms, spmv_n = float(run["fam_ms"][1]), int(run["fam_n"][1])
-    orth_ms, orth_n = float(run["fam_ms"][2]), int(run["fam_n"][2])
+    spmv_ms, spmv_n = float(prof["fam_ms"][1]), int(prof["fam_n"][1])
+    orth_ms, orth_n = float(prof["fam_ms"][2]), int(prof["fam_n"][2])
     # one block-Jacobi SpMV launch: 2x2 values (32 B FP64, 16 B FP32) + column index (4 B) per block, row
     # offsets, the input vector and the output once (16 B per node each), the 2x2 inverse (32 B per node)
     spmv_bytes = mesh.blocks * (20 if fp32 else 36) + 4 * (n + 1) + 16 * n * 2 + 32 * n
@@ -698,11 +711,11 @@ def run_transport(args, world, rank, local):
         traffic = TRANSPORT_SPMV_FP32_DRAM_BYTES_PER_BLOCK * mesh.blocks if fp32 else None
         kernels["spmv_block_jacobi_2x2"] = {"bound": "hbm", "achieved": a, "peak": hbm, "unit": "GB/s",
                                             "frac": a / hbm, "traffic": traffic, "launches": spmv_n,
-                                            "avg_ms": spmv_ms / spmv_n, "share": spmv_ms / ms,
+                                            "avg_ms": spmv_ms / spmv_n, "share": spmv_ms / prof["ms"],
                                             "algorithmic_bytes": spmv_bytes}
     if orth_n:
         kernels["krylov_orthogonalisation"] = {"launches": orth_n, "avg_ms": orth_ms / orth_n,
-                                               "share": orth_ms / ms}
+                                               "share": orth_ms / prof["ms"]}
     roof = dict(kernels.get("spmv_block_jacobi_2x2", {}))
     roof["kernel"] = "spmv_block_jacobi_2x2"
     roof["peak_kind"] = f"{peak_kind} hbm_gbs"
@@ -721,7 +734,9 @@ def run_transport(args, world, rank, local):
                    "l2": "inputs larger than L2 (L %.2f GB)" % (mesh.blocks * 32 / 1e9),
                    "parallelism": "replicas only" if world > 1 else "single GPU"},
         "gmres_iterations_per_step": its_per_step, "final_l2": timed_report["final_l2"],
-        "assembly_ms": run["assembly_ms"], "roofline": roof, "kernels": kernels, "fp64_gpu": fp64_leg,
+        "assembly_ms": run["assembly_ms"], "roofline": roof, "kernels": kernels,
+        "profile_pass": profile_pass(prof["ms"] / args.steps, int(prof["launches"]), int(run["launches"])),
+        "fp64_gpu": fp64_leg,
         "gpu_launches": int(run["launches"]), "clocks": run["clocks"],
         "e2e": {"value": replica_throughput(world, total_steps, e2e_ms), "unit": "time steps/s",
                 "h2d_bytes_per_step": (velocity.nbytes + mask.nbytes + n0.nbytes + nplus.nbytes) / total_steps,
@@ -909,6 +924,7 @@ def main():
     restart()
     ns.set_profiling(True)
     ns.profile(reset=True)
+    prof_launches = ns.launches()
     p0, p1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
     prof_ms = 0.0
     for k in range(args.warmup, total):
@@ -923,6 +939,7 @@ def main():
     orth_algo, orth_moved = prof_bytes["krylov_orthogonalisation"]
     spmv_counted = prof_bytes["spmv"][0]     # the per-tube solver counts the rows of open tubes only
     prof = ns.profile(reset=True)
+    prof_launches = ns.launches() - prof_launches
     ns.set_profiling(False)
 
     # e2e leg: same steps from the same state through the C ABI, inputs from pinned host memory, the
@@ -1219,9 +1236,8 @@ def main():
         "outlet_iterations_per_step": (float(np.mean([r.get("outlet_iterations", r.get("pressure_updates", 0))
                                                       for r in timed_reports])) if outlets else None),
         "roofline": roof, "kernels": kernels,
-        "profile_pass": {"ms_per_step": prof_ms / args.steps, "attributed_share": attributed,
-                         "note": "kernel families timed in a repeat of the timed steps; shares are of that "
-                                 "pass's duration"},
+        "profile_pass": dict(profile_pass(prof_ms / args.steps, prof_launches, int(launches)),
+                             attributed_share=attributed),
         "fp64_gpu": fp64_leg,
         "spmv_gbs": kernels.get(spmv_name, {}).get("achieved"),
         "gpu_launches": int(launches),
