@@ -280,6 +280,12 @@ int tfiga_ns_apply_dirichlet(tfiga_ns* ns, double* values, double* rhs);
  * (SolveGmres, Gmres.hpp:192-336): update = A^{-1} rhs. */
 int tfiga_ns_solve_linear(tfiga_ns* ns, double rtol, int32_t max_iterations, double* update,
 	int32_t* iterations, double* residual);
+/* Limits of the solves that run as one cooperative launch (systems whose Krylov basis fits the chip's shared memory; not
+ * while profiling).  iterations_per_launch (default 4096): a longer solve continues in a further launch, at the next
+ * restart.  wait_ns (default 4e9): the longest wall-clock wait at a barrier of the launch, which takes microseconds; when
+ * it runs out (0: always) the solve is done by separate launches from its start, and so are the handle's later ones
+ * until this is called again. */
+int tfiga_ns_set_solve_limits(tfiga_ns* ns, int32_t iterations_per_launch, int64_t wait_ns);
 /* One full Newton iteration: assemble, diagnostics, Dirichlet rows, norm and
  * convergence test, GMRES, state += update (iga_cuda.cu:956-1046).
  * initial_residual is the step's first residual norm (<0 on the first iteration). */

@@ -175,6 +175,7 @@ SIGNATURES = {
     "tfiga_ns_amg_info": (C.c_int, [C.c_void_p, C.POINTER(AmgInfo)]),
     "tfiga_ns_tangent_kernel": (C.c_int, [C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p]),
     "tfiga_ns_tangent_element_ms": (C.c_int, [C.c_void_p, C.c_void_p]),
+    "tfiga_ns_set_solve_limits": (C.c_int, [C.c_void_p, C.c_int32, C.c_int64]),
     "tfiga_ns_set_segments": (C.c_int, [C.c_void_p, C.c_void_p, C.c_int32]),
     "tfiga_ns_segment_status": (C.c_int, [C.c_void_p, C.c_void_p, C.c_void_p]),
     "tfiga_ns_boundary_flows": (C.c_int, [C.c_void_p, C.c_void_p, C.c_int32, C.c_void_p]),
@@ -398,6 +399,10 @@ class NavierStokes:
         it = C.c_int32(); res = C.c_double()
         check(lib().tfiga_ns_solve_linear(self._h, rtol, max_iterations, _p(u), C.byref(it), C.byref(res)))
         return u, it.value, res.value
+
+    def set_solve_limits(self, iterations_per_launch=4096, wait_ns=4_000_000_000):
+        """Limits of the solves in one cooperative launch (tfiga_ns_set_solve_limits)."""
+        check(lib().tfiga_ns_set_solve_limits(self._h, iterations_per_launch, wait_ns))
 
     def newton_iteration(self, initial_residual=-1.0) -> dict:
         r = NewtonReport()

@@ -399,6 +399,15 @@ int tfiga_ns_step_outlets_coupled(tfiga_ns* ns, tfiga_outlet* outlets, int32_t c
 	});
 }
 
+int tfiga_ns_set_solve_limits(tfiga_ns* ns, int32_t iterations_per_launch, int64_t wait_ns)
+{
+	return Guard([&] {
+		Require(ns != nullptr, "null handle");
+		Require(iterations_per_launch > 0 && wait_ns >= 0, "solve limits out of range");
+		ns->solver->SetSolveLimits(iterations_per_launch, wait_ns);
+	});
+}
+
 int tfiga_ns_set_segments(tfiga_ns* ns, const int64_t* node_offsets, int32_t count)
 {
 	return Guard([&] {

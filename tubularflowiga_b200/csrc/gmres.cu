@@ -478,8 +478,16 @@ bool Gmres::SolveResident(ResidentKrylov::Kind kind, const DevicePatternView& pa
 		problem.Z = Z_.get();
 		if (low_on_) problem.low = {low_.count, low_.ptr, low_.idx, low_.val, low_.coef};
 	}
+	// the start, for a solve whose barrier wait runs out (the CTAs did not get to run together in time): the separate
+	// launches, which wait for nothing, then solve from it, now and from here on
+	const size_t bytes = (size_t)n_*sizeof(double);
+	CudaCheck(cudaMemcpyAsync(tmp_.get(), problem.x, bytes, cudaMemcpyDeviceToDevice, stream_), "resident GMRES start");
 	const ResidentStatus status = resident_.Solve(problem, stream_, &launches_);
-	if (status.error == 4) Fail(-2, std::string(name)+": a grid barrier wait expired");
+	if (status.error == 4) {
+		CudaCheck(cudaMemcpyAsync(problem.x, tmp_.get(), bytes, cudaMemcpyDeviceToDevice, stream_),
+			"resident GMRES start");
+		return false;
+	}
 	if (status.error == 2)
 		Fail(-6, std::string(name)+(status.iterations ? " residual is not finite" : " initial residual is not finite"));
 	if (status.error == 1) Fail(-6, std::string(name)+" Hessenberg matrix is singular");

@@ -77,6 +77,10 @@ public:
 	// segment k's rows (for the profiler's byte counts of the masked SpMV).
 	void SetSegments(const std::vector<int64_t>& entry_offsets, const std::vector<int64_t>& blocks = {});
 	int segments() const { return segments_; }
+	void set_resident_limits(int iterations_per_launch, long long wait_ns)
+	{
+		resident_.SetLimits(iterations_per_launch, wait_ns);
+	}
 	// SolveFlexible with one Arnoldi process per segment sharing the SpMV and preconditioner launches:
 	// each segment its own Hessenberg matrix, rotations and tolerance rtol * ||b_k - A x0_k|| (the matrix
 	// and the preconditioner must not couple segments).  Converged when every segment meets its own;
@@ -134,7 +138,7 @@ private:
 
 	// One cooperative launch for the whole solve where the basis fits the chip's shared memory; direct
 	// launches otherwise, and while profiling (the families' events lie between kernels), with the
-	// learned stage, a pair collector or the flow lines.  False: not taken.
+	// learned stage, a pair collector or the flow lines.  False: not taken, or given up with x as it was.
 	bool SolveResident(ResidentKrylov::Kind kind, const DevicePatternView& pattern, const AmgResidentView* amg,
 		const std::vector<int64_t>& segments, ResidentProblem& problem, GmresResult& result, const char* name);
 	ResidentKrylov resident_;

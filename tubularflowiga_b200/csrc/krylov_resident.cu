@@ -24,8 +24,9 @@
 // shared coarse solve.
 //
 // Memory written by other CTAs in this launch is read with plain (coherent after the barrier's acquire)
-// loads, never through the read-only path.  Barrier waits are bounded: on expiry the status says so and
-// every CTA returns.
+// loads, never through the read-only path.  Barrier waits are bounded (ResidentKrylov's wait limit): a CTA whose wait
+// runs out says so in the status and returns, the others' waits run out in turn, and the caller solves by separate
+// launches.
 #include "krylov_resident.hpp"
 
 #include "block_row.cuh"
@@ -49,14 +50,13 @@ constexpr int kCoarseMax = 512;                // aggregates at most (a coarse v
 // AMG's arrays; a larger one is loaded to leave the L2 first, so that the vectors stay.  (82 MB batch: 3.65 ms a solve
 // streamed, 3.12 ms kept; 199 MB section: 7.75 ms streamed, 8.2 to 8.6 ms with 48 to 96 MB of it kept.)
 constexpr size_t kKeepBytes = (size_t)96 << 20;
-constexpr unsigned long long kWaitNs = 4000000000ull;
-constexpr int kIterationsPerLaunch = 4096;     // bounds one launch; a longer solve continues in the next
 
 struct Args {
 	ResidentProblem p;
 	int restart, slice, pieces, ctas, groups;
 	bool keep;                                 // the matrix stays in the L2
 	int max_cycles_iterations;
+	long long wait_ns;                         // limit of a barrier wait
 	const int32_t *cta_row, *cta_group, *group_cta, *agg_list, *agg_list_offsets;
 	// restriction: the nodes of every CTA by aggregate (part_nodes from part_start of its parts cta_parts ..), a
 	// partial sum per part; each aggregate's parts are part_list from part_offsets; aggregates by group
@@ -77,23 +77,25 @@ __device__ __forceinline__ double WarpSum(double v)
 	return v;
 }
 
-// Grid barrier on a counter that only grows; false when a wait ran out (in this or any CTA).
-__device__ __forceinline__ bool GridBarrier(unsigned* counter, unsigned target, int* expired)
+// Grid barrier on a counter that only grows; false when this CTA's wait ran out (`expired` is the CTA's own: the others
+// learn of it from their next wait).
+__device__ __forceinline__ bool GridBarrier(unsigned* counter, unsigned target, long long wait_ns, int* expired)
 {
 	__syncthreads();
 	if (threadIdx.x == 0) {
 		int bad = 0;
 		asm volatile("red.release.gpu.global.add.u32 [%0], 1;" :: "l"(counter) : "memory");
 		unsigned seen;
-		unsigned long long start = 0;
+		long long start = 0;
 		for (int spin = 0;; ++spin) {
 			asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(counter) : "memory");
 			if (seen >= target) break;
+			if (wait_ns == 0) { bad = 1; break; }
 			if ((spin & 255) == 255) {
-				unsigned long long now;
+				long long now;
 				asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(now));
 				if (start == 0) start = now;
-				else if (now-start > kWaitNs) { bad = 1; break; }
+				else if (now-start > wait_ns) { bad = 1; break; }
 			}
 		}
 		__threadfence();
@@ -213,7 +215,7 @@ __global__ void __launch_bounds__(kFlex ? kThreadsFlexible : kThreadsLeft, 1) Re
 	if (tid == 0) expired = 0;
 	for (int r = tid; r <= row1-row0; r += kThreads) rows[r] = a.p.pattern.row_offsets[row0+r];
 	__syncthreads();
-	auto barrier = [&]() { ++epoch; return GridBarrier(a.barrier, epoch*(unsigned)G, &expired); };
+	auto barrier = [&]() { ++epoch; return GridBarrier(a.barrier, epoch*(unsigned)G, a.wait_ns, &expired); };
 
 	// Own rows of A x into `piece`, one warp per (row, piece of its blocks); warps `skip` and up take part.
 	auto product = [&](const auto* values, const double* x, int skip, bool keep) {
@@ -936,7 +938,8 @@ ResidentStatus ResidentKrylov::Solve(const ResidentProblem& problem, cudaStream_
 	args.ctas = ctas_;
 	args.groups = groups_;
 	args.keep = keep_;
-	args.max_cycles_iterations = kIterationsPerLaunch;
+	args.max_cycles_iterations = iterations_per_launch_;
+	args.wait_ns = wait_ns_;
 	args.cta_row = cta_row_.get();
 	args.cta_group = cta_group_.get();
 	args.group_cta = group_cta_.get();
@@ -972,6 +975,7 @@ ResidentStatus ResidentKrylov::Solve(const ResidentProblem& problem, cudaStream_
 		total.iterations += host_->iterations;
 		total.error = host_->error;
 		total.residual = host_->residual;
+		if (total.error == 4) fits_ = false;
 		if (total.error || total.converged || total.iterations >= problem.max_iterations || host_->iterations == 0)
 			return total;
 		args.tolerance_in = tolerance_.get();

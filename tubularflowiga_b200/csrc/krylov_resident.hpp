@@ -66,8 +66,18 @@ public:
 	// (entry offsets, count + 1 values, or empty) are not those of the last call.
 	bool Prepare(Kind kind, const DevicePatternView& pattern, int restart, const std::vector<int64_t>& segments,
 		const AmgResidentView* amg, cudaStream_t stream);
-	// Runs the solve and waits for it.
+	// Runs the solve and waits for it.  After a status with error 4 the plan is off (Prepare returns false), and x holds
+	// whatever the CTAs had reached.
 	ResidentStatus Solve(const ResidentProblem& problem, cudaStream_t stream, long long* launches);
+	// Iterations after which a launch ends and the next one continues (checked between restart cycles), and the limit
+	// of a wait at a grid barrier (0: any wait runs out).  Four seconds of wall clock: a barrier takes microseconds.
+	// A plan that is off is made again.
+	void SetLimits(int iterations_per_launch, long long wait_ns)
+	{
+		iterations_per_launch_ = iterations_per_launch;
+		wait_ns_ = wait_ns;
+		planned_ = false;
+	}
 private:
 	void Plan(const DevicePatternView& pattern, const AmgResidentView* amg, cudaStream_t stream);
 	bool planned_ = false, fits_ = false;
@@ -76,6 +86,8 @@ private:
 	long long amg_version_ = -1;
 	int ctas_ = 0, groups_ = 1, restart_ = 0, slice_ = 0, pieces_ = 1, threads_ = 0;
 	bool keep_ = false;
+	int iterations_per_launch_ = 4096;
+	long long wait_ns_ = 4000000000ll;
 	size_t smem_ = 0;
 	DeviceArray<int32_t> cta_row_, cta_group_, group_cta_, agg_list_, agg_list_offsets_;
 	static constexpr int kTables = 7;

@@ -56,6 +56,10 @@ public:
 	// and each open segment's rhs is scaled to unit norm for the solve (its update scaled back after).
 	// The step converges when every segment passes (and the mass test holds).
 	void SetSegments(const int64_t* node_offsets, int count);
+	void SetSolveLimits(int iterations_per_launch, long long wait_ns)
+	{
+		gmres_.set_resident_limits(iterations_per_launch, wait_ns);
+	}
 	// After a Newton iteration: per segment 1 if it has passed its test in this step, and its residual.
 	void SegmentStatus(int32_t* done, double* residuals) const;
 	void Synchronize();
