@@ -137,7 +137,9 @@ typedef struct tfiga_ns_params {
 	 * Newton convergence rate can change.  Default 0 (off). */
 	double tangent_reuse_factor;   /* default 0 */
 	/* Tensor-core modes: how the tangent's basis values reach the tensor cores, and how the work is
-	 * spread.  The point kernel stores 72 numbers per quadrature point (18 KiB per element) in all of them.
+	 * spread.  The point kernel stores 72 numbers per quadrature point (18 KiB per element) in all of them; FUSED,
+	 * and AUTO, hold them for 2,048 elements at a time, made again before the tangent, where they would take more than
+	 * a quarter of the free memory.
 	 * TFIGA_TANGENT_COEFFICIENTS: an FP32 copy of the basis tables (80 KiB per element) is kept; a CTA per
 	 * element and row field;
 	 * TFIGA_TANGENT_ELEMENT: the same copy, two persistent CTAs per SM that take element after element;

@@ -85,13 +85,13 @@ void LaunchAssembleLarge(const DeviceMeshView& mesh, int first, int count, const
 	double* rhs, cudaStream_t stream);
 
 // ---- tangent_tc.cu -----------------------------------------------------
-// The tangent contracted on the tcgen05 tensor cores from the points' numbers (LaunchPointStream's packs32 of all
-// elements) and the basis values (phi32, the FP32 copy of Mesh::phi32, or phi when that is null), FP32
+// The tangent of the elements [first, first + count) contracted on the tcgen05 tensor cores from their points' numbers
+// (LaunchPointStream's packs32) and the basis values (phi32, the FP32 copy of Mesh::phi32, or phi when that is null), FP32
 // accumulation, ADDED into the FP32 values; status bit 1 set if an MMA completion wait expired.
 // operands: TC_OPERANDS_BF16, TC_OPERANDS_SPLIT (hi + lo BF16) or TC_OPERANDS_TF32.  persistent: two CTAs per SM
 // take (element, row field) after (element, row field), instead of a CTA for each.
 enum : int { TC_OPERANDS_BF16 = 0, TC_OPERANDS_SPLIT = 1, TC_OPERANDS_TF32 = 2 };
-void LaunchTangentTc(const DeviceMeshView& mesh, const float* phi32, const double* phi, const float* packs,
+void LaunchTangentTc(const DeviceMeshView& mesh, int first, int count, const float* phi32, const double* phi, const float* packs,
 	const int32_t* element_blocks, AssemblyParams params, float* values, int* status, int operands, bool persistent,
 	cudaStream_t stream);
 

@@ -87,10 +87,16 @@ NsSolver::NsSolver(Mesh& mesh, const tfiga_ns_params& params)
 		Fail(-1, "unknown tangent_kernel "+std::to_string(params.tangent_kernel));
 	tangent_kernel_ = params.tangent_kernel;
 	if (tensor_tangent()) {
-		const size_t regular = (size_t)mesh.regular_elements();
-		packs32_.Allocate(regular*kQuad*kPointNumbers);
-	}
-	if (tensor_tangent()) {
+		// The points' numbers of every element (18 KiB each), written by the residual pass.  The organisation for meshes
+		// that barely fit makes them a slab at a time instead where they would take more than a quarter of the free
+		// memory (so does AUTO, whose other organisations' FP32 tables, 80 KiB per element, do not fit then either).
+		// Residual and tangent of the 25,600-element tube: 9.04 ms whole, 10.04 in slabs.
+		const size_t numbers = (size_t)mesh.regular_elements()*kQuad*kPointNumbers;
+		size_t free_bytes = 0, total_bytes = 0;
+		CudaCheck(cudaMemGetInfo(&free_bytes, &total_bytes), "device memory");
+		packs_whole_ = tangent_kernel_ == TFIGA_TANGENT_COEFFICIENTS || tangent_kernel_ == TFIGA_TANGENT_ELEMENT
+			|| numbers*sizeof(float) <= free_bytes/4;
+		if (packs_whole_) packs32_.Allocate(numbers);
 		status_.Allocate(1);
 		status_.Zero(stream_);
 		CudaCheck(cudaMallocHost(reinterpret_cast<void**>(&pinned_status_), sizeof(int32_t)), "pinned status");
@@ -212,7 +218,8 @@ void NsSolver::AssembleResidualTc()
 	profiler_.End(stream_);
 	profiler_.Begin(Profiler::kResidual, stream_);
 	LaunchPointStream(mesh_.regular_view(), 0, (int)mesh_.regular_elements(), mesh_.phi(), mesh_.qdata(), state_.get(),
-		previous_.get(), {params_.density, params_.viscosity, params_.dt}, nullptr, packs32_.get(), rhs_.get(), stream_);
+		previous_.get(), {params_.density, params_.viscosity, params_.dt}, nullptr, packs_whole_ ? packs32_.get() : nullptr,
+		rhs_.get(), stream_);
 	LargeElements<float>(nullptr, rhs_.get());
 	profiler_.End(stream_);
 	profiler_.Begin(Profiler::kVector, stream_);
@@ -231,13 +238,47 @@ void NsSolver::LargeElements(T* values, double* rhs)
 	launches_ += 1;
 }
 
+namespace {
+
+// Elements per slab of points' numbers: 74 MB (FP64) that the L2 holds between the kernel that makes them and the one that
+// reads them.
+constexpr int kSlab = 2048;
+
+// The elements of a slab, its work array allocated on the first call: fewer where the memory does not suffice.
+template <class T>
+int SlabElements(DeviceArray<T>& packs, int count)
+{
+	for (int slab = std::min(kSlab, count); packs.size() == 0; slab /= 2) {
+		try {
+			packs.Allocate((size_t)slab*kQuad*kPointNumbers);
+		} catch (const Error& error) {
+			if (error.status != -8 || slab < 2) throw;
+		}
+	}
+	return (int)(packs.size()/(kQuad*kPointNumbers));
+}
+
+} // namespace
+
 void NsSolver::LaunchTangent(int organisation)
 {
+	const AssemblyParams prm{params_.density, params_.viscosity, params_.dt};
+	const DeviceMeshView view = mesh_.regular_view();
+	const int count = (int)mesh_.regular_elements();
+	const float* phi32 = organisation == TFIGA_TANGENT_FUSED ? nullptr : mesh_.phi32();
 	values32_.Zero(stream_);
-	LaunchTangentTc(mesh_.regular_view(), organisation == TFIGA_TANGENT_FUSED ? nullptr : mesh_.phi32(), mesh_.phi(),
-		packs32_.get(), mesh_.element_blocks(), {params_.density, params_.viscosity, params_.dt}, values32_.get(),
-		status_.get(), tc_operands(), organisation == TFIGA_TANGENT_ELEMENT, stream_);
-	launches_ += 1;
+	const int per = packs_whole_ || count == 0 ? count : SlabElements(packs32_, count);
+	for (int first = 0; first < count; first += per) {
+		const int slab = std::min(per, count-first);
+		if (!packs_whole_) {
+			LaunchPointStream(view, first, slab, mesh_.phi(), mesh_.qdata(), state_.get(), previous_.get(), prm, nullptr,
+				packs32_.get(), nullptr, stream_);
+			launches_ += 1;
+		}
+		LaunchTangentTc(view, first, slab, phi32, mesh_.phi(), packs32_.get(), mesh_.element_blocks(), prm, values32_.get(),
+			status_.get(), tc_operands(), organisation == TFIGA_TANGENT_ELEMENT, stream_);
+		launches_ += 1;
+	}
 }
 
 void NsSolver::AssembleTangentTc()
@@ -274,7 +315,7 @@ void NsSolver::AutotuneTangent()
 	const size_t need = (size_t)mesh_.regular_elements()*kFeatures*kQuad*kMaxBasis*sizeof(float);
 	size_t free_bytes = 0, total_bytes = 0;
 	CudaCheck(cudaMemGetInfo(&free_bytes, &total_bytes), "device memory");
-	if (!mesh_.has_phi32() && free_bytes < need+(size_t(2) << 30)) return;
+	if (!packs_whole_ || (!mesh_.has_phi32() && free_bytes < need+(size_t(2) << 30))) return;
 	const bool had = mesh_.has_phi32();
 	mesh_.phi32();
 	// (the last one's tangent, equal to the others' up to the order of the FP32 additions, is kept)
@@ -308,15 +349,12 @@ void NsSolver::AssembleResidual()
 
 void NsSolver::AssembleFp64(double* rhs)
 {
-	// in slabs of elements, whose points' numbers (36 KiB per element, 74 MB in all) share one workspace that the L2
-	// holds between the two kernels
-	constexpr int kSlab = 2048;
 	const int count = (int)mesh_.regular_elements();
 	const AssemblyParams prm{params_.density, params_.viscosity, params_.dt};
-	if (packs_.size() == 0) packs_.Allocate((size_t)std::min(kSlab, count)*kQuad*kPointNumbers);
+	const int per = count == 0 ? 0 : SlabElements(packs_, count);
 	values_.Zero(stream_);
-	for (int first = 0; first < count; first += kSlab) {
-		const int slab = std::min(kSlab, count-first);
+	for (int first = 0; first < count; first += per) {
+		const int slab = std::min(per, count-first);
 		LaunchPointStream(mesh_.regular_view(), first, slab, mesh_.phi(), mesh_.qdata(), state_.get(), previous_.get(), prm,
 			packs_.get(), nullptr, rhs, stream_);
 		LaunchAssembleTangent(mesh_.regular_view(), first, slab, mesh_.phi(), packs_.get(), mesh_.element_blocks(), prm,

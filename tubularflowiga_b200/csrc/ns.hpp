@@ -156,7 +156,8 @@ private:
 	int64_t n4_;
 	DeviceArray<double> values_, rhs_, state_, previous_, update_, traction_, velocity_bc_, pressure_bc_;
 	DeviceArray<float> values32_;
-	DeviceArray<float> packs32_;             // tensor-core tangent: the points' numbers of every element
+	DeviceArray<float> packs32_;             // tensor-core tangent: the points' numbers of every element or of a slab
+	bool packs_whole_ = false;
 	DeviceArray<double> packs_;              // FP64 tangent: the points' numbers of a slab of elements
 	int tangent_kernel_ = 0;                 // TFIGA_TANGENT_* in use
 	double tune_ms_[3] = {0.0, 0.0, 0.0};    // autotuner: coefficients, fused, element times

@@ -632,15 +632,22 @@ void LaunchMode(const DeviceMeshView& mesh, const float* phi32, const double* ph
 
 } // namespace
 
-void LaunchTangentTc(const DeviceMeshView& mesh, const float* phi32, const double* phi, const float* packs,
-	const int32_t* element_blocks, AssemblyParams params, float* values, int* status, int operands, bool persistent,
-	cudaStream_t stream)
+void LaunchTangentTc(const DeviceMeshView& mesh, int first, int count, const float* phi32, const double* phi,
+	const float* packs, const int32_t* element_blocks, AssemblyParams params, float* values, int* status, int operands,
+	bool persistent, cudaStream_t stream)
 {
+	// the arrays by element begin at `first`
+	DeviceMeshView view = mesh;
+	view.elements = count;
+	view.element_offsets += first;
+	element_blocks += (size_t)first*kMaxBasis*kMaxBasis;
+	const size_t tables = (size_t)first*kFeatures*kQuad*kMaxBasis;
 	if (phi32)
-		LaunchMode<false>(mesh, phi32, nullptr, packs, element_blocks, params, values, status, operands, persistent,
+		LaunchMode<false>(view, phi32+tables, nullptr, packs, element_blocks, params, values, status, operands, persistent,
 			stream);
 	else
-		LaunchMode<true>(mesh, nullptr, phi, packs, element_blocks, params, values, status, operands, persistent, stream);
+		LaunchMode<true>(view, nullptr, phi+tables, packs, element_blocks, params, values, status, operands, persistent,
+			stream);
 }
 
 } // namespace tfiga
