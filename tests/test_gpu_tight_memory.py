@@ -74,3 +74,62 @@ def test_points_numbers_in_slabs(api, section, kernel):
     finally:
         del held
         free_bytes()
+
+
+HOLE = 32768
+
+
+class Full:
+    """All device memory that cudaMalloc gives, down to pieces of 512 bytes, but for a hole of 32 KiB."""
+
+    def __init__(self):
+        import ctypes
+        self.runtime = ctypes.CDLL("libcudart.so.12")
+        self.runtime.cudaMalloc.argtypes = [ctypes.c_void_p, ctypes.c_size_t]
+        self.runtime.cudaFree.argtypes = [ctypes.c_void_p]
+        self.pieces = []
+        hole, size = self.take(HOLE), 1 << 37
+        while size >= 512:
+            pointer = self.take(size)
+            if pointer is None:
+                size //= 2
+            else:
+                self.pieces.append(pointer)
+        self.runtime.cudaFree(hole)
+
+    def take(self, size):
+        import ctypes
+        pointer = ctypes.c_void_p()
+        if self.runtime.cudaMalloc(ctypes.byref(pointer), size) == 0:
+            return pointer
+        self.runtime.cudaGetLastError()
+        return None
+
+    def close(self):
+        for p in self.pieces:
+            self.runtime.cudaFree(p)
+
+
+@pytest.mark.parametrize("kind", ["block-jacobi", "amg"])
+def test_solve_without_memory_for_its_plan(api, kind):
+    """A solve whose one-launch plan finds no memory (the triangular factor alone takes 33 KB) runs as separate launches,
+    which need none of the plan's arrays, and holds on to none of them."""
+    from tests.test_gpu_resident_limits import solve, system
+    ns, _ = system(kind)
+    ns.set_profiling(True)                  # separate launches: their arrays and code are there now
+    want, iterations, launches = solve(ns)
+    ns.set_profiling(False)
+    full = Full()
+    try:
+        update, _, separate = solve(ns)
+        hole = full.take(HOLE)
+        if hole is not None:
+            full.pieces.append(hole)
+    finally:
+        full.close()
+    assert launches > iterations and separate > iterations
+    assert rel(update, want) < 1e-7
+    assert hole is not None
+    ns.set_solve_limits()                   # plans anew
+    update, iterations, once = solve(ns)
+    assert once < iterations and rel(update, want) < 1e-7

@@ -478,8 +478,8 @@ bool Gmres::SolveResident(ResidentKrylov::Kind kind, const DevicePatternView& pa
 		problem.Z = Z_.get();
 		if (low_on_) problem.low = {low_.count, low_.ptr, low_.idx, low_.val, low_.coef};
 	}
-	// the start, for a solve whose barrier wait runs out (the CTAs did not get to run together in time): the separate
-	// launches, which wait for nothing, then solve from it, now and from here on
+	// the start, for a solve whose barrier wait runs out (the CTAs did not get to run together in time) or whose launch is
+	// refused: the separate launches, which wait for nothing, then solve from it, now and from here on
 	const size_t bytes = (size_t)n_*sizeof(double);
 	CudaCheck(cudaMemcpyAsync(tmp_.get(), problem.x, bytes, cudaMemcpyDeviceToDevice, stream_), "resident GMRES start");
 	const ResidentStatus status = resident_.Solve(problem, stream_, &launches_);

@@ -764,11 +764,21 @@ bool ResidentKrylov::Prepare(Kind kind, const DevicePatternView& pattern, int re
 	fits_ = false;
 	try {
 		Plan(pattern, amg, stream);
-	} catch (const Error& error) {
-		if (error.status != -8) throw;       // no memory for the work arrays: the separate launches need none of them
+	} catch (const Error&) {
+		// no memory for the work arrays or the kernel's code: the separate launches need neither
+		ReleaseArrays();
+		fits_ = false;
 	}
 	planned_ = true;
 	return fits_;
+}
+
+void ResidentKrylov::ReleaseArrays()
+{
+	for (auto* a : {&cta_row_, &cta_group_, &group_cta_, &agg_list_, &agg_list_offsets_, &status_}) a->Release();
+	for (auto& a : tables_) a.Release();
+	for (auto* a : {&partial_, &R_, &y_, &tolerance_, &coarse_part_}) a->Release();
+	flags_.Release();
 }
 
 void ResidentKrylov::Plan(const DevicePatternView& pattern, const AmgResidentView* amg, cudaStream_t stream)
@@ -965,8 +975,14 @@ ResidentStatus ResidentKrylov::Solve(const ResidentProblem& problem, cudaStream_
 	for (;;) {
 		status_.Zero(stream);
 		void* parameters[] = {&args};
-		CudaCheck(cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(KernelOf(kind_)), dim3(ctas_), dim3(threads_),
-			parameters, smem_, stream), "ResidentKrylovKernel");
+		if (cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(KernelOf(kind_)), dim3(ctas_), dim3(threads_),
+			parameters, smem_, stream) != cudaSuccess) {
+			// fewer CTAs than planned can run together here, or no memory for the launch
+			(void)cudaGetLastError();
+			total.error = 4;
+			fits_ = false;
+			return total;
+		}
 		if (launches) *launches += 1;
 		CudaCheck(cudaMemcpyAsync(host_, args.status, sizeof(ResidentStatus), cudaMemcpyDeviceToHost, stream),
 			"resident GMRES status");

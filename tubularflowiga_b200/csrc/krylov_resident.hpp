@@ -36,7 +36,7 @@ struct ResidentLowRank {
 // What the kernel reports to the host.
 struct ResidentStatus {
 	int converged, iterations;
-	int error;                               // 1 singular Hessenberg, 2 not finite, 4 a barrier wait ran out
+	int error;                               // 1 singular Hessenberg, 2 not finite, 4 a barrier wait ran out or no launch
 	unsigned barrier;                        // arrivals at the grid barriers of this launch
 	double residual;
 };
@@ -80,6 +80,7 @@ public:
 	}
 private:
 	void Plan(const DevicePatternView& pattern, const AmgResidentView* amg, cudaStream_t stream);
+	void ReleaseArrays();
 	bool planned_ = false, fits_ = false;
 	Kind kind_ = kLeft4;
 	std::vector<int64_t> segments_;
