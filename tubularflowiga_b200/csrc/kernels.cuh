@@ -91,9 +91,11 @@ void LaunchAssembleLarge(const DeviceMeshView& mesh, int first, int count, const
 // operands: TC_OPERANDS_BF16, TC_OPERANDS_SPLIT (hi + lo BF16) or TC_OPERANDS_TF32.  persistent: two CTAs per SM
 // take (element, row field) after (element, row field), instead of a CTA for each.
 enum : int { TC_OPERANDS_BF16 = 0, TC_OPERANDS_SPLIT = 1, TC_OPERANDS_TF32 = 2 };
-void LaunchTangentTc(const DeviceMeshView& mesh, int first, int count, const float* phi32, const double* phi, const float* packs,
-	const int32_t* element_blocks, AssemblyParams params, float* values, int* status, int operands, bool persistent,
-	cudaStream_t stream);
+// Loads the kernels of these operands, so that a first launch does not (between the autotuner's events, say).
+void LoadTangentTc(int operands);
+void LaunchTangentTc(const DeviceMeshView& mesh, int first, int count, const float* phi32, const double* phi,
+	const float* packs, const int32_t* element_blocks, AssemblyParams params, float* values, int* status, int operands,
+	bool persistent, cudaStream_t stream);
 
 // ---- sparse.cu ----------------------------------------------------------
 // Matrix values are FP64 or FP32 (T = double / float); vectors are FP64.

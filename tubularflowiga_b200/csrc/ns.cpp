@@ -309,6 +309,7 @@ void NsSolver::AutotuneTangent()
 		CudaCheck(cudaEventElapsedTime(&ms, ev[0], ev[1]), "event time");
 		return (double)ms;
 	};
+	LoadTangentTc(tc_operands());
 	tune_ms_[1] = timed(TFIGA_TANGENT_FUSED);
 	tangent_kernel_ = TFIGA_TANGENT_FUSED;
 	// the organisations with an FP32 copy of the basis tables, when it fits with 2 GiB to spare (or is there)

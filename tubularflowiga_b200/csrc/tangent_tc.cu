@@ -591,6 +591,16 @@ __global__ void __launch_bounds__(Threads(kFp64Tables), 2) TangentKernel(DeviceM
 		asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" :: "r"(tmem), "r"((uint32_t)kTmemCols));
 }
 
+// Loads the kernel and allows its shared memory (bytes returned).
+template <int kMode, bool kFp64Tables>
+int Configure()
+{
+	const int bytes = (int)sizeof(TangentShared<kFp64Tables>)+1024;
+	CudaCheck(cudaFuncSetAttribute(TangentKernel<kMode, kFp64Tables>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+		bytes), "tangent shared memory");
+	return bytes;
+}
+
 template <int kMode, bool kFp64Tables>
 void Launch(const DeviceMeshView& mesh, const float* phi32, const double* phi64, const float* packs,
 	const int32_t* element_blocks, AssemblyParams params, float* values, int* status, bool persistent,
@@ -599,9 +609,7 @@ void Launch(const DeviceMeshView& mesh, const float* phi32, const double* phi64,
 	const long long items = 4LL*mesh.elements;
 	if (items == 0) return;
 	if (items > 0x7fffffffLL) Fail(-7, "too many elements for one tangent launch");
-	const int bytes = (int)sizeof(TangentShared<kFp64Tables>)+1024;
-	CudaCheck(cudaFuncSetAttribute(TangentKernel<kMode, kFp64Tables>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-		bytes), "tangent shared memory");
+	const int bytes = Configure<kMode, kFp64Tables>();
 	long long grid = items;
 	if (persistent) {
 		int device = 0, sms = 0;
@@ -631,6 +639,13 @@ void LaunchMode(const DeviceMeshView& mesh, const float* phi32, const double* ph
 }
 
 } // namespace
+
+void LoadTangentTc(int operands)
+{
+	if (operands == TC_OPERANDS_SPLIT) Configure<kModeSplit, false>(), Configure<kModeSplit, true>();
+	else if (operands == TC_OPERANDS_TF32) Configure<kModeTf32, false>(), Configure<kModeTf32, true>();
+	else Configure<kModeBf16, false>(), Configure<kModeBf16, true>();
+}
 
 void LaunchTangentTc(const DeviceMeshView& mesh, int first, int count, const float* phi32, const double* phi,
 	const float* packs, const int32_t* element_blocks, AssemblyParams params, float* values, int* status, int operands,
