@@ -1,8 +1,9 @@
 """The 4x4-block product in every form that the mesh's size selects, and at every remainder of a row's blocks.
 
 Rows are shared by four warps up to 2,368 of them, by two up to 4,736, and have one warp above; a matrix of more than
-96 MiB is streamed past the L2.  The meshes lie in these ranges (asserted, so that a change of the rule shows), and the
-rows of a thinned mesh have from 1 to some 90 blocks.  Products agree with the host's to 1e-14 of the largest entry-wise
+96 MiB is streamed past the L2, and in FP32 the rows' remainders are taken by twos from 10,065 to 14,208 rows.  The
+meshes lie in these ranges (asserted, so that a change of the rule shows), and the rows of a thinned mesh have from 1 to
+some 90 blocks.  Products agree with the host's to 1e-14 of the largest entry-wise
 sum of magnitudes and 1e-12 of each entry's own (sums of up to 1,372 products of FP64 numbers in another order).
 """
 import numpy as np
@@ -12,6 +13,7 @@ pytestmark = pytest.mark.gpu
 
 STREAM = 96 << 20
 FOUR, TWO = 2368, 4736
+PAIRS = range(10065, 14209)
 
 
 def products(flat, reduced, seed):
@@ -47,15 +49,19 @@ def check(y, expected, magnitude):
     assert (np.abs(y - expected) <= 1e-12 * magnitude + 1e-300).all()
 
 
-@pytest.mark.parametrize("core, ring, layers, reduced, parts, streamed", [
-    (4, 1, 30, False, 4, False), (5, 1, 70, False, 2, False), (3, 1, 250, False, 1, False), (6, 1, 100, False, 1, True),
-    (4, 1, 30, True, 4, False), (5, 1, 70, True, 2, False), (6, 1, 70, True, 1, False), (6, 1, 140, True, 1, True)])
-def test_product_of_every_form(core, ring, layers, reduced, parts, streamed):
-    from tubularflowiga_b200 import meshgen
-    flat = meshgen.straight_tube(1.5e-3, 2e-4 * layers, core, ring, layers).mesh
+@pytest.mark.parametrize("core, ring, layers, reduced, parts, streamed, pairs", [
+    (4, 1, 30, False, 4, False, False), (5, 1, 70, False, 2, False, False), (3, 1, 250, False, 1, False, False),
+    (6, 1, 100, False, 1, True, False), (6, 1, 140, False, 1, True, False),
+    (4, 1, 30, True, 4, False, False), (5, 1, 70, True, 2, False, False), (6, 1, 70, True, 1, False, False),
+    (6, 1, 136, True, 1, True, False), (6, 1, 140, True, 1, True, True), (5, 2, 180, True, 1, True, True),
+    (8, 2, 100, True, 1, True, False)])
+def test_product_of_every_form(core, ring, layers, reduced, parts, streamed, pairs):
+    from perf import cases
+    flat = cases.long_tube(core, ring, layers, cases.LAYER).mesh
     y, expected, magnitude, size = products(flat, reduced, layers)
     assert parts == (4 if flat.nodes <= FOUR else 2 if flat.nodes <= TWO else 1)
     assert streamed == (size > STREAM)
+    assert pairs == (reduced and streamed and flat.nodes in PAIRS)
     check(y, expected, magnitude)
 
 

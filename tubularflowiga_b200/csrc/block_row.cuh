@@ -55,8 +55,8 @@ __device__ __forceinline__ double QuadRowSum(double s)
 	return s;
 }
 
-// Part `part` of kParts of (A x)[4*row + r], in lanes with lane & 3 == r.
-template <class T, int kParts, bool kStream>
+// Part `part` of kParts of (A x)[4*row + r], in lanes with lane & 3 == r.  kPairs: a row's remainder by twos.
+template <class T, int kParts, bool kStream, bool kPairs>
 __device__ __forceinline__ double RowBlockDot(const DevicePatternView& p, const T* __restrict__ values,
 	const double* __restrict__ x, int row, int part, int lane)
 {
@@ -81,24 +81,24 @@ __device__ __forceinline__ double RowBlockDot(const DevicePatternView& p, const 
 			s = a[u].Dot(__ldg(v), __ldg(v+1), s);
 		}
 	}
-	if constexpr (sizeof(T) == 4 && kParts == 1 && kStream) {
-		// What is left, in one round of predicated loads: 64 registers and half the warps, but two or three round trips
-		// to memory fewer.  It pays where values come from HBM (FP32, 10,716 rows of 166 blocks, 109 MiB: 37.0 us with the
-		// loop below, 28.8 so, 30.9 with a block per lane; 29,145 rows, 358 MiB: 73.9, 69.7 and 80.0) and not from the
-		// L2 (8,241 rows, 68 MiB: 14.4 us with the loop, 16.3 so).
-		int c[kUnroll];
-		BlockRow<T> a[kUnroll];
-		#pragma unroll
-		for (int u = 0; u < kUnroll; ++u) c[u] = b+8*u < hi ? __ldg(p.columns+b+8*u) : -1;
-		#pragma unroll
-		for (int u = 0; u < kUnroll; ++u)
-			if (c[u] >= 0) a[u].template Load<kStream>(values, (size_t)(b+8*u), r);
-		#pragma unroll
-		for (int u = 0; u < kUnroll; ++u)
-			if (c[u] >= 0) {
-				const double2* v = reinterpret_cast<const double2*>(x+4*(size_t)c[u]);
-				s = a[u].Dot(__ldg(v), __ldg(v+1), s);
-			}
+	if constexpr (kPairs) {
+		// what is left by twos, in predicated loads: half the round trips to memory of the loop below
+		#pragma unroll 1
+		for (; b-(lane >> 2) < hi; b += 16) {
+			int c[2];
+			BlockRow<T> a[2];
+			#pragma unroll
+			for (int u = 0; u < 2; ++u) c[u] = b+8*u < hi ? __ldg(p.columns+b+8*u) : -1;
+			#pragma unroll
+			for (int u = 0; u < 2; ++u)
+				if (c[u] >= 0) a[u].template Load<kStream>(values, (size_t)(b+8*u), r);
+			#pragma unroll
+			for (int u = 0; u < 2; ++u)
+				if (c[u] >= 0) {
+					const double2* v = reinterpret_cast<const double2*>(x+4*(size_t)c[u]);
+					s = a[u].Dot(__ldg(v), __ldg(v+1), s);
+				}
+		}
 	} else {
 		for (; b < hi; b += 8) {
 			const double2* v = reinterpret_cast<const double2*>(x+4*(size_t)__ldg(p.columns+b));

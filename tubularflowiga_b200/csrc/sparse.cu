@@ -16,8 +16,8 @@ constexpr int kSpmvWarps = 8;        // warps per CTA
 
 // y = [D^-1] (scale * A x): inverse, scale, stop and the segments (node_seg, seg_stop: rows of stopped segments keep
 // their old y) are optional.
-template <class T, int kParts, bool kStream>
-__global__ void __launch_bounds__(32*kSpmvWarps) SpmvKernel(DevicePatternView p, const T* __restrict__ values,
+template <class T, int kParts, bool kStream, bool kPairs>
+__global__ void __launch_bounds__(32*kSpmvWarps, kPairs ? 6 : 0) SpmvKernel(DevicePatternView p, const T* __restrict__ values,
 	const double* __restrict__ inverse, const double* __restrict__ x, const double* __restrict__ scale,
 	double* __restrict__ y, const int* __restrict__ stop, const int32_t* __restrict__ node_seg,
 	const int* __restrict__ seg_stop)
@@ -28,7 +28,7 @@ __global__ void __launch_bounds__(32*kSpmvWarps) SpmvKernel(DevicePatternView p,
 	int row = blockIdx.x*kRows+warp/kParts;
 	const auto skipped = [&](int r) { return r >= p.nodes || (seg_stop != nullptr && seg_stop[node_seg[r]]); };
 	double sum = 0.0;
-	if (!skipped(row)) sum = RowBlockDot<T, kParts, kStream>(p, values, x, row, warp%kParts, lane);
+	if (!skipped(row)) sum = RowBlockDot<T, kParts, kStream, kPairs>(p, values, x, row, warp%kParts, lane);
 	if constexpr (kParts > 1) {
 		// the parts of a row, four lanes per row in the first warp
 		__shared__ double parts[kSpmvWarps][4];
@@ -59,6 +59,12 @@ constexpr size_t kSpmvStreamBytes = (size_t)96 << 20;
 // Warps that fill the chip (64 on each of 148 SMs): rows are split while their parts do not exceed them (cylinder of
 // 1,681 rows, FP64: 14.4 us with a warp per row, 6.2 with four; 14,645 rows: 39 us with one, 41 with two).
 constexpr int kSpmvFill = 64*148;
+// FP32 products with one warp per row: past a full wave of warps the chip is left to a few of them, and their last blocks,
+// eight at a time, are what is waited for.  The remainder by twos takes 40 registers, six CTAs per SM instead of eight,
+// and is used from 17/16 of a wave to one and a half.  (10,716 rows of 166 blocks, 109 MiB: 37.4 us without, 30.8 with,
+// 30.9 with a block per lane; 11,745 rows, 142 MiB: 39.3, 36.9, 38.6; 9,576 rows: 28.7, 29.7, 28.8.  With other work on
+// the chip, three streams at once, both take the same: 18.8 and 23.6 us a product.)
+constexpr int kSpmvPairsFrom = kSpmvFill+kSpmvFill/16, kSpmvPairsTo = kSpmvFill+kSpmvFill/2;
 
 template <class T>
 void SpmvLaunch(const DevicePatternView& p, const T* values, const double* inverse, const double* x,
@@ -70,10 +76,12 @@ void SpmvLaunch(const DevicePatternView& p, const T* values, const double* inver
 		kernel<<<(unsigned)((p.nodes+rows-1)/rows), 32*kSpmvWarps, 0, stream>>>(p, values, inverse, x, scale, y, stop,
 			node_seg, seg_stop);
 	};
-	if (4LL*p.nodes <= kSpmvFill) launch(SpmvKernel<T, 4, false>, 4);
-	else if (2LL*p.nodes <= kSpmvFill) launch(SpmvKernel<T, 2, false>, 2);
-	else if ((size_t)p.blocks*16*sizeof(T) <= kSpmvStreamBytes) launch(SpmvKernel<T, 1, false>, 1);
-	else launch(SpmvKernel<T, 1, true>, 1);
+	if (4LL*p.nodes <= kSpmvFill) launch(SpmvKernel<T, 4, false, false>, 4);
+	else if (2LL*p.nodes <= kSpmvFill) launch(SpmvKernel<T, 2, false, false>, 2);
+	else if ((size_t)p.blocks*16*sizeof(T) <= kSpmvStreamBytes) launch(SpmvKernel<T, 1, false, false>, 1);
+	else if (sizeof(T) == 4 && p.nodes > kSpmvPairsFrom && p.nodes <= kSpmvPairsTo) {
+		if constexpr (sizeof(T) == 4) launch(SpmvKernel<T, 1, true, true>, 1);
+	} else launch(SpmvKernel<T, 1, true, false>, 1);
 	LaunchCheck("SpmvKernel");
 }
 
