@@ -478,16 +478,12 @@ bool Gmres::SolveResident(ResidentKrylov::Kind kind, const DevicePatternView& pa
 		problem.Z = Z_.get();
 		if (low_on_) problem.low = {low_.count, low_.ptr, low_.idx, low_.val, low_.coef};
 	}
-	// the start, for a solve whose barrier wait runs out (the CTAs did not get to run together in time) or whose launch is
-	// refused: the separate launches, which wait for nothing, then solve from it, now and from here on
-	const size_t bytes = (size_t)n_*sizeof(double);
-	CudaCheck(cudaMemcpyAsync(tmp_.get(), problem.x, bytes, cudaMemcpyDeviceToDevice, stream_), "resident GMRES start");
+	problem.start = tmp_.get();
+	problem.fields = fields_;
 	const ResidentStatus status = resident_.Solve(problem, stream_, &launches_);
-	if (status.error == 4) {
-		CudaCheck(cudaMemcpyAsync(problem.x, tmp_.get(), bytes, cudaMemcpyDeviceToDevice, stream_),
-			"resident GMRES start");
-		return false;
-	}
+	// a barrier wait that ran out (the CTAs did not get to run together in time) or a launch that was refused: the separate
+	// launches, which wait for nothing, solve from the same start, now and from here on
+	if (status.error == 4) return false;
 	if (status.error == 2)
 		Fail(-6, std::string(name)+(status.iterations ? " residual is not finite" : " initial residual is not finite"));
 	if (status.error == 1) Fail(-6, std::string(name)+" Hessenberg matrix is singular");

@@ -440,9 +440,16 @@ __global__ void __launch_bounds__(kFlex ? kThreadsFlexible : kThreadsLeft, 1) Re
 
 	int iterations = 0;
 	double tolerance = 0.0;
+	// x as it was, for a caller who has to start again; kept by every CTA once the first barrier is passed, and x changes
+	// only after that.  (The left-preconditioned solves are fewer and longer, and short of registers: the host keeps it.)
+	if constexpr (kFlex)
+		if (!a.tolerance_in)
+			for (int k = tid; k < len; k += kThreads) a.p.start[lo+k] = a.p.x[lo+k];
 	residual();
 	publish(0);
 	if (!barrier()) return give_up(iterations);
+	if constexpr (kFlex)
+		if (cta == 0 && tid == 0) a.status->kept = 1;
 	for (int cycle = 0;; ++cycle) {
 		// beta of the own group, then whether every group meets its tolerance (each CTA sums them all)
 		const double beta = group_norm(g0, g1);
@@ -972,6 +979,20 @@ ResidentStatus ResidentKrylov::Solve(const ResidentProblem& problem, cudaStream_
 	args.status = reinterpret_cast<ResidentStatus*>(status_.get());
 	args.barrier = &args.status->barrier;
 	ResidentStatus total{};
+	const auto copy = [&](double* to, const double* from) {
+		CudaCheck(cudaMemcpyAsync(to, from, problem.entries()*sizeof(double), cudaMemcpyDeviceToDevice, stream),
+			"resident GMRES start");
+	};
+	if (kind_ == kLeft2 || kind_ == kLeft2Fp32 || kind_ == kLeft4) {
+		copy(problem.start, problem.x);
+		total.kept = 1;
+	}
+	const auto give_up = [&]() {
+		if (total.kept) copy(problem.x, problem.start);
+		total.error = 4;
+		fits_ = false;
+		return total;
+	};
 	for (;;) {
 		status_.Zero(stream);
 		void* parameters[] = {&args};
@@ -979,9 +1000,7 @@ ResidentStatus ResidentKrylov::Solve(const ResidentProblem& problem, cudaStream_
 			parameters, smem_, stream) != cudaSuccess) {
 			// fewer CTAs than planned can run together here, or no memory for the launch
 			(void)cudaGetLastError();
-			total.error = 4;
-			fits_ = false;
-			return total;
+			return give_up();
 		}
 		if (launches) *launches += 1;
 		CudaCheck(cudaMemcpyAsync(host_, args.status, sizeof(ResidentStatus), cudaMemcpyDeviceToHost, stream),
@@ -991,7 +1010,8 @@ ResidentStatus ResidentKrylov::Solve(const ResidentProblem& problem, cudaStream_
 		total.iterations += host_->iterations;
 		total.error = host_->error;
 		total.residual = host_->residual;
-		if (total.error == 4) fits_ = false;
+		total.kept |= host_->kept;
+		if (total.error == 4) return give_up();
 		if (total.error || total.converged || total.iterations >= problem.max_iterations || host_->iterations == 0)
 			return total;
 		args.tolerance_in = tolerance_.get();

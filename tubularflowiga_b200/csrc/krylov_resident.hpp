@@ -38,6 +38,7 @@ struct ResidentStatus {
 	int converged, iterations;
 	int error;                               // 1 singular Hessenberg, 2 not finite, 4 a barrier wait ran out or no launch
 	unsigned barrier;                        // arrivals at the grid barriers of this launch
+	int kept;                                // 1 once x's start is kept in full
 	double residual;
 };
 
@@ -48,6 +49,7 @@ struct ResidentProblem {
 	const void* residual_values = nullptr;   // operator of the true residual
 	const double* rhs = nullptr;
 	double* x = nullptr;
+	double* start = nullptr;                 // scratch of x's size
 	const double* inverse = nullptr;         // left block-Jacobi
 	AmgResidentView amg;                     // right preconditioner of the flexible solve
 	ResidentLowRank low;
@@ -55,6 +57,8 @@ struct ResidentProblem {
 	void* V = nullptr;                       // basis: [restart + 1][n]
 	double rtol = 0.0, tolerance_floor = 0.0;
 	int max_iterations = 0;
+	int fields = 4;
+	std::size_t entries() const { return (std::size_t)fields*pattern.nodes; }
 };
 
 // Rows of every CTA, groups (independent segments) and work arrays of a matrix; laid out once.
@@ -66,8 +70,8 @@ public:
 	// (entry offsets, count + 1 values, or empty) are not those of the last call.
 	bool Prepare(Kind kind, const DevicePatternView& pattern, int restart, const std::vector<int64_t>& segments,
 		const AmgResidentView* amg, cudaStream_t stream);
-	// Runs the solve and waits for it.  After a status with error 4 the plan is off (Prepare returns false), and x holds
-	// whatever the CTAs had reached.
+	// Runs the solve and waits for it.  After a status with error 4 the plan is off (Prepare returns false) and x is as it
+	// was before.
 	ResidentStatus Solve(const ResidentProblem& problem, cudaStream_t stream, long long* launches);
 	// Iterations after which a launch ends and the next one continues (checked between restart cycles), and the limit
 	// of a wait at a grid barrier (0: any wait runs out).  Four seconds of wall clock: a barrier takes microseconds.
