@@ -40,9 +40,12 @@ Legs of one run (rank 0 prints one JSON line):
   e2e       the same steps again, from the same starting state, through the
             C ABI with pinned host inputs (inlet Dirichlet values) and the
             state read back every step.
-  roofline  per-kernel CUDA-event timing of the timed region: the tensor-core
-            (or FP64) assembly, SpMV, the AMG V-cycle and the Krylov
-            orthogonalisation (HBM-bound); the dominant one by share.
+  roofline  per-kernel CUDA-event timing of an instrumented repeat of the timed
+            steps: the tensor-core (or FP64) assembly, SpMV, the AMG V-cycle and
+            the Krylov orthogonalisation (HBM-bound); the dominant one by share.
+            Instrumented linear solves are separate launches: on the small
+            meshes (c1, c2-100), whose timed solves take one launch each, these
+            families are not those of the timed steps ("profile_pass").
   fp64_gpu  (mixed only) the plain FP64 GPU solver on the warm-up steps from
             the same initial state (same outlet coupling), run with the fixed
             1e-8 tolerance and in the mixed arm's forcing mode; the faster of

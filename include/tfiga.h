@@ -146,7 +146,8 @@ typedef struct tfiga_ns_params {
 	 * TFIGA_TANGENT_FUSED: no copy, the FP64 tables are converted on the way;
 	 * TFIGA_TANGENT_AUTO: the first tangent assembly times the three (those with the copy when its memory
 	 * is free) and keeps the fastest; the fused one otherwise.
-	 * All give the same tangent up to the order of the FP32 additions. */
+	 * All give the same tangent up to the order of the FP32 additions.  The numbers of a point are computed in FP64 and
+	 * rounded to FP32; their products with the basis values are FP32, then rounded to the operands' type. */
 	int32_t tangent_kernel;        /* default TFIGA_TANGENT_AUTO */
 } tfiga_ns_params;
 
@@ -329,8 +330,9 @@ int tfiga_ns_amg_info(tfiga_ns* ns, tfiga_amg_info* info);
  * test is then taken per tube, relative to the tube's own first residual of the step, and a tube that
  * passes is frozen for the rest of the step (its rows of the linear system carry a zero rhs); the
  * linear solves run one FGMRES per tube over shared launches (each tube its own Arnoldi process,
- * Hessenberg matrix and tolerance, stopping on its own; the AMG preconditioner only; each Arnoldi step
- * replayed from a CUDA graph captured on its first use, except while profiling), each open
+ * Hessenberg matrix and tolerance, stopping on its own; the AMG preconditioner only; in one cooperative
+ * launch where the Krylov bases fit the chip's shared memory, else each Arnoldi step replayed from a CUDA
+ * graph captured on its first use; neither while profiling), each open
  * tube's rhs scaled to unit norm and its update scaled back; the step converges when every tube has
  * passed. */
 int tfiga_ns_set_segments(tfiga_ns* ns, const int64_t* node_offsets, int32_t count);
@@ -372,7 +374,9 @@ int tfiga_ns_stream(tfiga_ns* ns, void** stream);
  * Galerkin coarse operator, dense coarse inverse), 6 the Newton loop's own
  * vector work (residual and Jacobian zeroing, traction, convergence
  * diagnostics, Dirichlet rows, norms, the state update, device outlet
- * coupling, per-segment tests). */
+ * coupling, per-segment tests).  While it is on, linear solves run as separate
+ * launches, those too that otherwise take one cooperative launch
+ * (tfiga_ns_set_solve_limits): the families describe those kernels. */
 #define TFIGA_PROFILE_FAMILIES 7
 int tfiga_ns_set_profiling(tfiga_ns* ns, int enable);
 /* Totals since the last reset: milliseconds and launch counts per family. */
@@ -593,7 +597,8 @@ int tfiga_transport_apply_preconditioner(tfiga_transport* transport, const doubl
 int tfiga_transport_info(const tfiga_transport* transport, double* assembly_ms, int32_t* steps, int64_t* launches);
 /* The handle's CUDA stream (a cudaStream_t). */
 int tfiga_transport_stream(tfiga_transport* transport, void** stream);
-/* Per-family device timing as tfiga_ns_set_profiling / tfiga_ns_profile:
+/* Per-family device timing as tfiga_ns_set_profiling / tfiga_ns_profile (GMRES
+ * by separate launches while it is on):
  * family 1 SpMV (P c and the block-Jacobi SpMV of GMRES), 2 Krylov
  * orthogonalisation; the others stay 0. */
 int tfiga_transport_set_profiling(tfiga_transport* transport, int enable);
