@@ -17,10 +17,11 @@
 // the product.  m16n8k4 and not k16: scalar FP64 work of the builders queues behind the products on the same
 // pipe, 32 cycles each instead of 128.  Rows, columns and CTAs past the element's own function
 // count are skipped: elements at patch boundaries have 18 to 48 functions, and on the benchmark's meshes
-// nen^2 is 40 to 65 % of 64^2.  The FP64 pipe bounds it.  The kernel it replaces (one CTA per SM, 8 x 8
+// nen^2 is 40 to 65 % of 64^2.  The FP64 tensor pipe bounds it (55 % of its cycles on the cylinder; the rest are the
+// latency of a warp's products and the barrier of a chunk).  The kernel it replaces (one CTA per SM, 8 x 8
 // register tiles of scalar products over all 64 x 256 entries, the point state recomputed for each row
 // field) took 34.5 ms for the 12,800-element section and 3.4 ms for the 1,280-element cylinder; this one takes
-// 12.6 and 0.88 ms, 63 % of the FP64 pipe's time at 64 products per cycle and SM.
+// 12.6 and 0.88 ms, 60 and 53 % of what the FP64 tensor pipe can do at the measured 63 products per cycle and SM.
 #include "common.hpp"
 #include "kernels.cuh"
 #include "vms_point.cuh"
