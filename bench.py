@@ -208,6 +208,13 @@ def replica_throughput(world, steps, ms):
     return world * steps / (ms / 1e3)
 
 
+def residual_pass_bytes(mesh, numbers):
+    """Bytes of a residual pass: the FP64 basis values of every element's own functions (5 features at 64 points) and
+    the point data (64 x 11 doubles) read and, with `numbers`, the tangent's 72 FP32 numbers per point written (the
+    fused organisation's pass does not write them where it makes them in slabs: left out there, a lower bound)."""
+    return int(mesh.element_offsets[-1]) * 5 * 64 * 8 + mesh.elements * (64 * 11 * 8 + (72 * 64 * 4 if numbers else 0))
+
+
 def profile_pass(ms_per_step, launches, timed_launches):
     """What the kernel figures were taken from: a repeat of the timed steps with events between the kernels."""
     return {"ms_per_step": ms_per_step, "gpu_launches": launches, "timed_gpu_launches": timed_launches,
@@ -1166,10 +1173,7 @@ def main():
                              "avg_ms": asm_ms / asm_n, "share": asm_ms / prof_ms,
                              "peak_note": "nominal B200 FP64 (no measured FP64 peak on this pool)"}
     if res_n:
-        # FP64 residual (+ the tangent's numbers in the tensor-core modes): per element it reads the FP64
-        # basis tables (5 x 64 x 64 doubles) and the point data (64 x 11 doubles) and, in the tensor-core
-        # modes, writes 72 numbers per point (72 x 64 floats)
-        rbytes = tube.mesh.elements * (5 * 64 * 64 * 8 + 64 * 11 * 8 + (72 * 64 * 4 if mixed else 0))
+        rbytes = residual_pass_bytes(tube.mesh, mixed and tangent_info["kernel"] != "fused")
         a = rbytes / (res_ms / res_n * 1e-3) / 1e9
         kernels["residual_point"] = {"bound": "hbm", "achieved": a, "peak": hbm, "unit": "GB/s", "frac": a / hbm,
                                      "traffic": None, "launches": res_n, "avg_ms": res_ms / res_n,
